@@ -4,7 +4,7 @@
 // blocks, how many atom images per block, how long the z-lines are) and on the GPU:
 //   * prj_chunk   : blocks of one (image, source) list per projection CTA (the cubes-per-CTA
 //                   schedule of the projection: longer chunks amortize the pipeline start and
-//                   the coefficient atomics, shorter ones balance the load)   {8, 16, 32}
+//                   the coefficient atomics, shorter ones balance the load)   {12, 24, 40}
 //   * add_blocks  : consecutive blocks per CTA of the FP32 addition        {8, 16, 32}
 //   * local_variant: FP32 local kernel on rows with one-step-ahead loads, on plain rows, on
 //                   y-pencils, or on y-pencils with staged neighbour cubes     {0, 1, 2, 3}
@@ -61,7 +61,7 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
     float ms = 0;
     if (dp.nAI > 0 && dp.nCols > 0) {
         uint32_t best = dp.prj_chunk; float tbest = 1e30f;
-        for (uint32_t c : {8u, 16u, 32u}) {
+        for (uint32_t c : {12u, 24u, 40u}) {
             dp.prj_chunk = c;
             if (!build_prj_items(hp, dp) || !time_part<T>(dp, 1, y, x, ci, st, ms)) return false;
             std::snprintf(line, sizeof(line), "projector chunk %2u blocks: %.3f ms\n", c, ms); report += line;

@@ -31,6 +31,18 @@ struct DeviceBuffer {
 
 template <typename T> T *dptr(DeviceBuffer const &b) { return (T*)b.ptr; }
 
+// work item of the projection: positions [first, first + count) of the block list of one (image,
+// source) pair; the items of a pair form a group (position g_pos of g_count, ticket counters
+// 4 g_id ..., partial sums from row g_row on)
+struct PrjItem {
+    uint64_t first;
+    uint32_t count, coeff, src, lmax;          // coeff: first coefficient of the image
+    uint32_t g_pos, g_count, g_id, g_row;
+};
+constexpr uint32_t kMaxPrjItem = 40;           // positions per item at most
+// slot of a list position with its flags: last cube of its x-line, last line of its z-slab
+constexpr uint32_t kLineEnd = 1u << 30, kSlabEnd = 1u << 31, kSlotMask = kLineEnd - 1;
+
 struct DevicePlan {
     bool uploaded = false;       // plan geometry on the device
     bool values_dirty = true;    // potential / matrices / phases need re-upload
@@ -45,7 +57,7 @@ struct DevicePlan {
     bool fused_local = false;    // all directions use the 9-point stencil: fused kernel
     uint32_t max_zline = 0;      // cubes in the longest z-line
     // schedule parameters, set by the autotuner (autotune.cu) or left at these defaults
-    uint32_t prj_chunk = 16;         // blocks per projection work item
+    uint32_t prj_chunk = 0;          // blocks per projection work item (0: by the plan's size)
     uint32_t add_blocks = 16;        // blocks per CTA of the FP32 addition
     int local_variant = 2;           // FP32: 0 rows with one-step-ahead loads, 1 plain rows, 2 pencils, 3 staged pencils
     bool local64_pencils = true;     // FP64: pencils with the planes on two threads, else the row kernel
@@ -75,12 +87,15 @@ struct DevicePlan {
     DeviceBuffer dev_error;      // int: first error code recorded by a kernel (0: none)
     bool use_tc = true;          // FP32 projector on the tensor cores (else SIMT)
     struct ImageGroup { uint32_t count = 0; DeviceBuffer images; } img_group[8];  // images by basis size
-    // SIMT projection work items by basis size: (image, source, first, last) list positions,
-    // each at most kPrjChunk blocks, so that long block lists are spread over many CTAs
-    // items8 adds the item's group (the items of one (image, source) pair): first item, count,
-    // group index, first partial-sum slot; tickets[group] counts finished items (deterministic
-    // fixed-order sum of the partials by the last one, projector_simt.cu)
-    struct PrjItems { uint32_t count = 0, part_items = 0; DeviceBuffer items, items8, tickets; } prj_items[8];
+    // work items of the generic projection kernel by basis size: (image, source, first, last) list
+    // positions, each at most 16 blocks
+    struct PrjItems { uint32_t count = 0; DeviceBuffer items; } prj_items[8];
+    // the projection along lines (projector_line.cuh): items of every (image, source) pair, one
+    // record {block, slot and flags, mask} per list position, and the slots' tables as
+    // [dir][point][order] with 8 bytes per value (FP32: the value twice), the orders padded to even
+    struct PrjLine { uint32_t count = 0; size_t part_rows = 0; DeviceBuffer items, tickets; } prj_line;
+    DeviceBuffer prj_rec, line_tab64, line_tab32;
+    uint32_t nslots = 0;
     DeviceBuffer prj_part;       // partial projection sums of multi-item groups
     // batch plans (GreenPlan::replicate): npairs (energy, k-point) pairs of nsrc_pair sources each
     uint32_t npairs = 1, nsrc_pair = 0;
@@ -111,11 +126,13 @@ uint64_t launches_so_far();
 bool upload_values(GreenPlan const &hp, DevicePlan &dp);
 // projection work items (image, source, up to dp.prj_chunk consecutive blocks of its list)
 bool build_prj_items(GreenPlan const &hp, DevicePlan &dp);
+// a table [slot][order][dir][point] of the plan's slots in the layout of the line kernels
+bool make_line_table(DevicePlan const &dp, double const *slot_H, DeviceBuffer &t64, DeviceBuffer *t32, cudaStream_t st);
 // chooses the schedule parameters of the action for this plan by timing them (autotune.cu)
 template <typename T>
 bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string &report);
 bool ensure_dyadic_scratch(DevicePlan &dp, size_t elem_bytes);
-// partial-sum buffer of the deterministic SIMT projection for reals of elem_bytes
+// partial-sum buffer of the deterministic projection for reals of elem_bytes
 bool ensure_prj_part(DevicePlan &dp, size_t elem_bytes);
 
 // the action y = (H - E S) x on real_t = double or float
@@ -154,6 +171,11 @@ bool launch_add_tc(DevicePlan &dp, float *y, uint16_t const *colIndex, cudaStrea
 // both stage blocks with 16-byte copies and need 16-byte aligned x and y
 bool simt_projector_supported(DevicePlan const &dp, void const *x, void const *y, size_t real_bytes);
 template <typename T> bool launch_project_simt(DevicePlan &dp, T const *x, cudaStream_t st);
+// the projection along lines with the given tables (every coefficient of an active source is written)
+bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const *tab, cudaStream_t st);
+bool launch_project_line(DevicePlan &dp, double *apc, double const *x, void const *tab, cudaStream_t st);
+bool prepare_line_kernels32();
+bool prepare_line_kernels64();
 template <typename T> bool launch_add_simt(DevicePlan &dp, T *y, uint16_t const *colIndex, cudaStream_t st);
 
 } // namespace a43g

@@ -64,10 +64,22 @@ std::vector<int32_t> neighbour_table(GreenPlan const &hp) {
     return nbr;
 }
 
+// slot_H [slot][order][dir][point] as [slot][dir][point][order], the orders padded to lp; the FP32
+// table holds every value twice (a pair of columns)
+__global__ void k_line_table(double *t64, float2 *t32, double const *slot_H, size_t n, int nu, int lp) {
+    size_t const k = size_t(blockIdx.x)*blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    int const m = int(k % lp), di = int(k/lp % 12);
+    double const h = (m < nu) ? slot_H[(k/lp/12*nu + m)*12 + di] : 0.0;
+    t64[k] = h;
+    if (t32) t32[k] = make_float2(float(h), float(h));
+}
+
 } // namespace
 
 bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
-    if (!prepare_simt_kernels() || !prepare_tc_kernels() || !prepare_local_kernels()) return false;
+    if (!prepare_simt_kernels() || !prepare_line_kernels32() || !prepare_line_kernels64() || !prepare_tc_kernels() ||
+        !prepare_local_kernels()) return false;
     dp.nnzb = uint32_t(hp.nnzb()); dp.nRows = hp.nRows; dp.nCols = hp.nCols;
     dp.nAtoms = hp.nAtoms; dp.nAI = hp.nAtomImages;
     dp.ncoeffI = uint32_t(hp.ncoeff_images()); dp.ncoeffA = uint32_t(hp.ncoeff_atoms());
@@ -130,6 +142,25 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
     if (!put(dp.slot_H, hp.slot_H) || !put(dp.slot_mask, hp.slot_mask)) return false;
     if (!put(dp.slot_H32, std::vector<float>(hp.slot_H.begin(), hp.slot_H.end()))) return false;
     if (!put(dp.prj_slot, hp.prj_slot) || !put(dp.add_slot, hp.add_slot)) return false;
+    {   // tables of the line kernels (FP32: every value twice, a pair of columns) and their records
+        dp.nslots = uint32_t(hp.slot_mask.size());
+        if (!make_line_table(dp, dptr<double>(dp.slot_H), dp.line_tab64, &dp.line_tab32, nullptr)) return false;
+        if (hp.slot_mask.size() > kSlotMask) { set_error("too many projector slots"); return false; }
+        std::vector<uint32_t> rec(4*pc.size());
+        size_t k = 0;
+        for (auto const &c : hp.SHOprj)
+            for (uint32_t a = 0; a + 1 < c.start.size(); ++a)
+                for (uint32_t p = c.start[a]; p < c.start[a + 1]; ++p, ++k) {
+                    float const *here = &hp.rowCubePos[4*size_t(hp.rowindx[c.col[p]])];
+                    float const *next = (p + 1 < c.start[a + 1]) ? &hp.rowCubePos[4*size_t(hp.rowindx[c.col[p + 1]])] : nullptr;
+                    bool const slab = !next || next[2] != here[2], line = slab || next[1] != here[1];
+                    uint64_t const m = hp.slot_mask[hp.prj_slot[k]];
+                    rec[4*k + 0] = c.col[p];
+                    rec[4*k + 1] = hp.prj_slot[k] | (line ? kLineEnd : 0u) | (slab ? kSlabEnd : 0u);
+                    rec[4*k + 2] = uint32_t(m); rec[4*k + 3] = uint32_t(m >> 32);
+                }
+        if (!put(dp.prj_rec, rec)) return false;
+    }
     {   // one 16-byte record per addition pair, so the kernel needs no dependent index loads
         std::vector<uint32_t> info(4*size_t(hp.SHOadd.nnz()), 0u);
         for (size_t k = 0; k < hp.SHOadd.nnz(); ++k) {
@@ -184,43 +215,63 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
 }
 
 bool build_prj_items(GreenPlan const &hp, DevicePlan &dp) {
-    uint32_t const chunk = std::max<uint32_t>(1, dp.prj_chunk);
-    std::vector<uint32_t> items[8], items8[8];
-    uint32_t groups[8] = {0}, parts[8] = {0};
+    constexpr uint32_t kGenericChunk = 16;
+    size_t npos = 0;
+    for (auto const &c : hp.SHOprj) npos += c.nnz();
+    // positions per item: enough items for about 12 CTAs per SM (two CTAs per item at least), since
+    // small plans would leave SMs idle, and as many as an item's tables in
+    // shared memory allow
+    uint32_t chunk = dp.prj_chunk;
+    if (0 == chunk) chunk = uint32_t(std::min<size_t>(kMaxPrjItem, std::max<size_t>(8, 2*npos/(148*12))));
+    chunk = std::min(chunk, kMaxPrjItem);
+    std::vector<uint32_t> items[8];
+    std::vector<PrjItem> line;
+    uint32_t groups = 0;
+    size_t rows = 0;
+    uint64_t off = 0;
     for (uint32_t s = 0; s < hp.nCols; ++s) {
         auto const &c = hp.SHOprj[s];
-        if (c.start.empty()) continue;
         for (uint32_t a = 0; a < hp.nAtomImages; ++a) {
             int const L = hp.AtomImageLmax[a];
-            uint32_t const k0 = c.start[a], k1 = c.start[a + 1];
-            if (k0 >= k1) continue;
-            uint32_t const n = (k1 - k0 + chunk - 1)/chunk, first = uint32_t(items[L].size()/4);
-            uint32_t const part = (n > 1) ? parts[L] : 0u;
-            for (uint32_t k = k0; k < k1; k += chunk) {
-                uint32_t const it[4] = {a, s, k, std::min(k + chunk, k1)};
+            uint32_t const k0 = c.start.empty() ? 0 : c.start[a], k1 = c.start.empty() ? 0 : c.start[a + 1];
+            for (uint32_t k = k0; k < k1; k += kGenericChunk) {
+                uint32_t const it[4] = {a, s, k, std::min(k + kGenericChunk, k1)};
                 items[L].insert(items[L].end(), it, it + 4);
-                uint32_t const it8[8] = {a, s, k, std::min(k + chunk, k1), first, n, groups[L], part};
-                items8[L].insert(items8[L].end(), it8, it8 + 8);
             }
-            ++groups[L];
-            if (n > 1) parts[L] += n;
+            // a pair without blocks has one empty item, which writes its zero coefficients
+            uint32_t const len = k1 - k0, n = std::max(1u, (len + chunk - 1)/chunk);
+            for (uint32_t i = 0; i < n; ++i) {
+                uint64_t const b = k0 + uint64_t(len)*i/n, e = k0 + uint64_t(len)*(i + 1)/n;
+                line.push_back(PrjItem{off + b, uint32_t(e - b), hp.AtomImageStarts[a], s, uint32_t(L), i, n,
+                                       groups, uint32_t(rows)});
+            }
+            ++groups;
+            if (n > 1) rows += size_t(n)*nsho(L);
         }
+        off += c.col.size();
     }
     for (int L = 0; L < 8; ++L) {
-        auto &g = dp.prj_items[L];
-        g.count = uint32_t(items[L].size()/4);
-        g.part_items = parts[L];
-        if (!put(g.items, items[L]) || !put(g.items8, items8[L])) return false;
-        if (!put(g.tickets, std::vector<uint32_t>(std::max<uint32_t>(groups[L], 1), 0u))) return false;
+        dp.prj_items[L].count = uint32_t(items[L].size()/4);
+        if (!put(dp.prj_items[L].items, items[L])) return false;
     }
+    dp.prj_line.count = uint32_t(line.size());
+    dp.prj_line.part_rows = rows;
+    return put(dp.prj_line.items, line) && put(dp.prj_line.tickets, std::vector<uint32_t>(4*size_t(groups), 0u));
+}
+
+bool make_line_table(DevicePlan const &dp, double const *slot_H, DeviceBuffer &t64, DeviceBuffer *t32, cudaStream_t st) {
+    int const nu = dp.table_stride/12, lp = (dp.lmax_max | 1) + 1;
+    size_t const n = size_t(dp.nslots)*12*std::max(lp, 0);
+    if (nu < 1 || 0 == n) return true;
+    if (!t64.alloc(n*8) || (t32 && !t32->alloc(n*8))) return false;
+    k_line_table<<<unsigned((n + 255)/256), 256, 0, st>>>(dptr<double>(t64), t32 ? dptr<float2>(*t32) : nullptr, slot_H, n, nu, lp);
+    count_launch();
+    A43G_CUDA_TRY(cudaGetLastError());
     return true;
 }
 
 bool ensure_prj_part(DevicePlan &dp, size_t elem_bytes) {
-    size_t n = 16;
-    for (int L = 0; L < 8; ++L)
-        n = std::max(n, size_t(dp.prj_items[L].part_items)*size_t(((L + 1)*(L + 2)*(L + 3))/6)*128*elem_bytes);
-    return dp.prj_part.alloc(n);
+    return dp.prj_part.alloc(std::max<size_t>(16, dp.prj_line.part_rows*128*elem_bytes));
 }
 
 bool upload_values(GreenPlan const &hp, DevicePlan &dp) {

@@ -1,0 +1,12 @@
+// FP32 instantiations of the line-factorized projector (projector_line.cuh).
+#include "projector_line.cuh"
+
+namespace a43g {
+
+bool prepare_line_kernels32() { return line::prepare<float>(); }
+
+bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const *tab, cudaStream_t st) {
+    return line::launch_project<float>(dp, apc, x, tab, st);
+}
+
+} // namespace a43g

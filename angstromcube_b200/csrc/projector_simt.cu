@@ -1,22 +1,17 @@
-// Projector contraction of the action on the CUDA cores (FP32 and FP64), sum-factorized
-// (include/green_dyadic.hxx:112-288 projection, :325-518 addition).
+// Addition of the action on the CUDA cores (FP32 and FP64), sum-factorized
+// (include/green_dyadic.hxx:325-518), and the launches of the projection along lines.
 //
 // The projector functions are separable on the spherical mask,
 //     P_(ix,iy,iz)(x, y, z) = H_ix(x) H_iy(y) H_iz(z)   for points inside the projection radius,
 // so one (block, image) pair costs 64*(L+1) + 16*(L+1)(L+2)/2 + 4*nSHO fused multiply-adds per
 // column instead of 64*nSHO for the dense product (944 instead of 3584 at numax 5).
 //
-// Both kernels keep the 1D tables of the current (image, row) slot and the per-thread partial
-// sums in registers (loops fully unrolled for the basis size L), one thread per (real/imaginary
-// plane, right-hand-side column):
-//   * projection: one CTA per work item (image, source, up to 16 blocks of its list); the
-//     blocks stream through a double-buffered shared-memory stage filled with cp.async
-//     (16-byte copies, so x must be 16-byte aligned), and the partial coefficients of the item
-//     are added to the zeroed image coefficients with one atomic per coefficient;
-//   * addition: one CTA per block b, summing the contributions of all images near b in
-//     registers and updating y[b] once; the coefficients of the next image are staged in shared
-//     memory with cp.async while the current one is applied (16-byte copies of rows that start
-//     on 512-byte boundaries of the plan's coefficient array).
+// One CTA per run of blocks, one thread per (real/imaginary plane, column) with the 1D tables of
+// the current (image, row) slot and the point sums in registers (loops fully unrolled for the
+// basis size L): the contributions of all images near a block are summed and y is updated once;
+// the coefficients of the next image are staged in shared memory with cp.async while the current
+// one is applied (16-byte copies of rows that start on 512-byte boundaries of the plan's
+// coefficient array).
 #include "device.cuh"
 
 #include <algorithm>
@@ -29,7 +24,6 @@ constexpr int kBlk = 8192;            // floats per block: 2 planes x 64 points 
 constexpr int kThreads = 128;
 
 __host__ __device__ constexpr int nsho_of(int L) { return ((L + 1)*(L + 2)*(L + 3))/6; }
-__host__ __device__ constexpr int n2_of(int L) { return ((L + 1)*(L + 2))/2; }
 
 __device__ __forceinline__ uint32_t smem_addr(void const *p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
@@ -66,172 +60,11 @@ __device__ __forceinline__ float fmat(float a, float b, float c) { return fmaf(a
 __device__ __forceinline__ double fmat(double a, double b, double c) { return fma(a, b, c); }
 
 // CTAs per SM the kernels are compiled for (FP64 needs twice the registers and shared memory)
-template <typename T> struct Occ { static constexpr int project = 3, add = 2; };
-template <> struct Occ<double> { static constexpr int project = 1, add = 1; };
+template <typename T> struct Occ { static constexpr int add = 2; };
+template <> struct Occ<double> { static constexpr int add = 1; };
 
 __device__ __forceinline__ void cp_async8(void *dst, void const *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(smem_addr(dst)), "l"(src) : "memory");
-}
-
-// ---------------------------------------------------------------- projection
-
-// Work item w = (image a, source s, list positions [k0, k1)) of group (first, count): the items of
-// one (image, source) pair.  A group of one item writes its coefficients directly; otherwise
-// every item stores its partial sums in part[w] and the last item of the group to finish (ticket
-// counter) adds the partials in item order, so the result does not depend on the order in which
-// the items ran, and resets the counter for the next call.
-// ZS threads share a column and split its z-planes (FP64: one CTA of 128 threads per SM would
-// leave one warp per scheduler); their partial coefficients are added in a fixed order at the end.
-template <typename T, int L, int ZS = int(sizeof(T))/4>
-__global__ void __launch_bounds__(kThreads*ZS, Occ<T>::project)
-sho_project_simt_kernel(T *__restrict__ apc, T const *__restrict__ x, uint32_t nrhs,
-                       uint32_t const *__restrict__ items, uint32_t const *__restrict__ prj_col,
-                       uint64_t const *__restrict__ prj_coloff, uint32_t const *__restrict__ prj_slot,
-                       T const *__restrict__ slot_H, uint64_t const *__restrict__ slot_mask, int stride,
-                       uint32_t const *__restrict__ img_starts, uint8_t const *__restrict__ active,
-                       T *__restrict__ part, uint32_t *__restrict__ tickets)
-{
-    constexpr int NS = nsho_of(L), N2 = n2_of(L);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *xs = reinterpret_cast<T*>(smem_raw);           // [2][kBlk]
-    uint32_t const *item = items + 8*size_t(blockIdx.x);
-    uint32_t const a = item[0], s = item[1], k0 = item[2], k1 = item[3];
-    uint32_t const g_first = item[4], g_count = item[5], g_id = item[6], g_part = item[7];
-    if (active && !active[s]) return;                 // uniform: a retired source
-    constexpr int NT = kThreads*ZS, NZ = 4/ZS;         // threads, z-planes per thread
-    int const tid = threadIdx.x, zh = tid/kThreads, reim = (tid >> 6) & 1, j = tid & 63;
-    uint64_t const off = prj_coloff[s];
-
-    __shared__ __align__(16) T tbuf[2][(L + 1)*12];       // 1D tables of the staged blocks' slots
-    __shared__ uint64_t mbuf[2];                           // and their masks
-    // block, table and mask of list position k go to shared memory ahead of use; the block and
-    // slot indices are loaded one position earlier still
-    auto stage = [&](uint32_t b, uint32_t slot, int buf) {
-        char const *src = reinterpret_cast<char const*>(x + size_t(b)*kBlk);
-        char *dst = reinterpret_cast<char*>(xs + buf*kBlk);
-#pragma unroll
-        for (int r = 0; r < kBlk*int(sizeof(T))/(16*NT); ++r) {
-            int const o = (r*NT + tid)*16;
-            cp_async16(dst + o, src + o);
-        }
-        constexpr int TE = 16/int(sizeof(T));          // table elements per 16-byte copy
-        if (tid < (L + 1)*12/TE) cp_async16(&tbuf[buf][tid*TE], slot_H + size_t(slot)*stride + tid*TE);
-        if (tid == NT - 1) cp_async8(&mbuf[buf], slot_mask + slot);
-    };
-
-    T acc[NS];
-#pragma unroll
-    for (int i = 0; i < NS; ++i) acc[i] = T(0);
-
-    stage(prj_col[off + k0], prj_slot[off + k0], 0);
-    cp_async_commit();
-    uint32_t nb = 0, ns = 0;
-    if (k0 + 1 < k1) { nb = prj_col[off + k0 + 1]; ns = prj_slot[off + k0 + 1]; }
-    int buf = 0;
-    for (uint32_t k = k0; k < k1; ++k, buf ^= 1) {
-        if (k + 1 < k1) stage(nb, ns, buf ^ 1);
-        cp_async_commit();
-        if (k + 2 < k1) { nb = prj_col[off + k + 2]; ns = prj_slot[off + k + 2]; }   // for the next iteration
-        cp_async_wait1();                            // block k has landed (this thread's copies)
-        __syncthreads();                             // ... and everybody else's
-        Tables<T, L> t;
-        t.load(tbuf[buf]);
-        // the x-functions of the slot in registers (FP64 reads the other tables in place)
-        T tx[L + 1][4];
-#pragma unroll
-        for (int ix = 0; ix <= L; ++ix)
-#pragma unroll
-            for (int xx = 0; xx < 4; ++xx) tx[ix][xx] = t(ix, 0, xx);
-        uint64_t const mask = mbuf[buf];
-        T const *xb = xs + buf*kBlk + reim*4096 + j;
-#pragma unroll
-        for (int zl = 0; zl < NZ; ++zl) {
-            int const z = zh*NZ + zl;
-            if (0 == ((mask >> (16*z)) & 0xffffu)) continue;     // uniform per thread: plane outside the sphere
-            T byx[N2];
-#pragma unroll
-            for (int i = 0; i < N2; ++i) byx[i] = T(0);
-#pragma unroll
-            for (int yy = 0; yy < 4; ++yy) {
-                T ax[L + 1];
-#pragma unroll
-                for (int i = 0; i <= L; ++i) ax[i] = T(0);
-#pragma unroll
-                for (int xx = 0; xx < 4; ++xx) {
-                    int const p = (z*4 + yy)*4 + xx;
-                    T const v = ((mask >> p) & 1u) ? xb[p*64] : T(0);
-#pragma unroll
-                    for (int ix = 0; ix <= L; ++ix) ax[ix] = fmat(v, tx[ix][xx], ax[ix]);
-                }
-#pragma unroll
-                for (int iy = 0, iyx = 0; iy <= L; ++iy) {
-                    T const hy = t(iy, 1, yy);
-#pragma unroll
-                    for (int ix = 0; ix <= L - iy; ++ix, ++iyx) byx[iyx] = fmat(ax[ix], hy, byx[iyx]);
-                }
-            }
-#pragma unroll
-            for (int iz = 0, sho = 0; iz <= L; ++iz) {
-                T const hz = t(iz, 2, z);
-#pragma unroll
-                for (int iy = 0; iy <= L - iz; ++iy) {
-                    int const iyx = iy*(2*L + 3 - iy)/2;
-#pragma unroll
-                    for (int ix = 0; ix <= L - iz - iy; ++ix, ++sho) acc[sho] = fmat(byx[iyx + ix], hz, acc[sho]);
-                }
-            }
-        }
-        __syncthreads();                             // buffer buf is free for block k + 2
-    }
-    if constexpr (ZS > 1) {
-        // the partial sums of the other z-planes, through the (now free) block stage, added in
-        // the order of the planes
-        cp_async_wait0();
-        __syncthreads();
-        if (zh > 0) {
-#pragma unroll
-            for (int sho = 0; sho < NS; ++sho) xs[(size_t(zh - 1)*NS + sho)*128 + reim*64 + j] = acc[sho];
-        }
-        __syncthreads();
-        if (zh > 0) return;
-        for (int h = 1; h < ZS; ++h) {
-#pragma unroll
-            for (int sho = 0; sho < NS; ++sho) acc[sho] += xs[(size_t(h - 1)*NS + sho)*128 + reim*64 + j];
-        }
-    }
-    T *out = apc + (size_t(img_starts[a])*nrhs + s)*128 + reim*64 + j;
-    if (1 == g_count) {
-#pragma unroll
-        for (int sho = 0; sho < NS; ++sho) out[size_t(sho)*nrhs*128] = acc[sho];
-        return;
-    }
-    // partial sums of this item: part[(g_part + position in group)][sho][128]
-    uint32_t const q = blockIdx.x - g_first;
-    T *mine = part + (size_t(g_part) + q)*NS*128 + reim*64 + j;
-#pragma unroll
-    for (int sho = 0; sho < NS; ++sho) mine[size_t(sho)*128] = acc[sho];
-    __threadfence();                                  // partials visible before the ticket
-    __shared__ uint32_t ticket;
-    if constexpr (ZS > 1) {
-        // the remaining threads of the first z-group only (the others have returned)
-        asm volatile("bar.sync 1, %0;" :: "n"(kThreads) : "memory");
-        if (0 == tid) ticket = atomicAdd(&tickets[g_id], 1u);
-        asm volatile("bar.sync 1, %0;" :: "n"(kThreads) : "memory");
-    } else {
-        __syncthreads();
-        if (0 == tid) ticket = atomicAdd(&tickets[g_id], 1u);
-        __syncthreads();
-    }
-    if (ticket + 1 != g_count) return;                // uniform: not the last item of the group
-    __threadfence();
-    T const *pg = part + size_t(g_part)*NS*128 + reim*64 + j;
-#pragma unroll 4
-    for (int sho = 0; sho < NS; ++sho) {
-        T sum = T(0);
-        for (uint32_t i = 0; i < g_count; ++i) sum += __ldcg(pg + (size_t(i)*NS + sho)*128);
-        out[size_t(sho)*nrhs*128] = sum;
-    }
-    if (0 == tid) tickets[g_id] = 0u;                 // ready for the next call
 }
 
 // ---------------------------------------------------------------- addition
@@ -425,19 +258,6 @@ template <typename T> T const *simt_table(DevicePlan const &dp);
 template <> float const *simt_table<float>(DevicePlan const &dp) { return dptr<float>(dp.slot_H32); }
 template <> double const *simt_table<double>(DevicePlan const &dp) { return dptr<double>(dp.slot_H); }
 
-template <typename T, int L>
-void launch_project_L(DevicePlan &dp, T const *x, cudaStream_t st) {
-    auto const &g = dp.prj_items[L];
-    if (0 == g.count) return;
-    constexpr int smem = 2*kBlk*int(sizeof(T));         // double-buffered block stage
-    sho_project_simt_kernel<T, L><<<g.count, kThreads*(int(sizeof(T))/4), smem, st>>>(
-        dptr<T>(dp.apc), x, dp.nCols, dptr<uint32_t>(g.items8), dptr<uint32_t>(dp.prj_col),
-        dptr<uint64_t>(dp.prj_coloff), dptr<uint32_t>(dp.prj_slot), simt_table<T>(dp),
-        dptr<uint64_t>(dp.slot_mask), dp.table_stride, dptr<uint32_t>(dp.img_starts),
-        dp.retire ? dptr<uint8_t>(dp.src_active) : nullptr, dptr<T>(dp.prj_part), dptr<uint32_t>(g.tickets));
-    count_launch();
-}
-
 template <typename T, int LMAX>
 void launch_add_L(DevicePlan &dp, T *y, uint16_t const *colIndex, cudaStream_t st) {
     constexpr int smem = (2*nsho_of(LMAX)*128 + kBlk)*int(sizeof(T));
@@ -453,8 +273,6 @@ void launch_add_L(DevicePlan &dp, T *y, uint16_t const *colIndex, cudaStream_t s
 
 template <typename T, int L>
 void set_smem_attributes() {
-    cudaFuncSetAttribute(sho_project_simt_kernel<T, L>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         2*kBlk*int(sizeof(T)));
     cudaFuncSetAttribute(sho_add_simt_kernel<T, L, int(sizeof(T))/4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (2*nsho_of(L)*128 + kBlk)*int(sizeof(T)));
     if (sizeof(T) == 8)
@@ -485,18 +303,8 @@ bool simt_projector_supported(DevicePlan const &dp, void const *x, void const *y
 
 template <typename T>
 bool launch_project_simt(DevicePlan &dp, T const *x, cudaStream_t st) {
-    // every (image, source) pair with blocks is written by its items; images without blocks of a
-    // source keep zero coefficients
     if (!ensure_prj_part(dp, sizeof(T))) return false;
-    A43G_CUDA_TRY(cudaMemsetAsync(dp.apc.ptr, 0, size_t(dp.ncoeffI)*dp.nCols*128*sizeof(T), st));
-    launch_project_L<T, 0>(dp, x, st); launch_project_L<T, 1>(dp, x, st);
-    launch_project_L<T, 2>(dp, x, st); launch_project_L<T, 3>(dp, x, st);
-    launch_project_L<T, 4>(dp, x, st); launch_project_L<T, 5>(dp, x, st);
-    if constexpr (sizeof(T) == 4) {
-        launch_project_L<T, 6>(dp, x, st); launch_project_L<T, 7>(dp, x, st);
-    }
-    A43G_CUDA_TRY(cudaGetLastError());
-    return true;
+    return launch_project_line(dp, dptr<T>(dp.apc), x, sizeof(T) == 8 ? dp.line_tab64.ptr : dp.line_tab32.ptr, st);
 }
 
 // (FP64 up to numax 5: its two coefficient stages and y fit 227 KB of shared memory)
