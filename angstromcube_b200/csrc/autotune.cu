@@ -5,7 +5,6 @@
 //   * prj_chunk   : blocks of one (image, source) list per projection CTA (the cubes-per-CTA
 //                   schedule of the projection: longer chunks amortize the pipeline start and
 //                   the coefficient atomics, shorter ones balance the load)   {12, 24, 40}
-//   * add_blocks  : consecutive blocks per CTA of the FP32 addition        {8, 16, 32}
 //   * local_variant: FP32 local kernel on rows with one-step-ahead loads, on plain rows, on
 //                   y-pencils, or on y-pencils with staged neighbour cubes     {0, 1, 2, 3}
 //   * use_tc      : FP32 projector on the tensor cores (3xTF32) or on the CUDA cores
@@ -70,14 +69,6 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
         dp.prj_chunk = best;
         if (!build_prj_items(hp, dp)) return false;
         if (sizeof(T) == 4) {
-            uint32_t bestb = dp.add_blocks; tbest = 1e30f;
-            for (uint32_t c : {8u, 16u, 32u}) {
-                dp.add_blocks = c;
-                if (!time_part<T>(dp, 1, y, x, ci, st, ms)) return false;
-                std::snprintf(line, sizeof(line), "addition %2u blocks per CTA: %.3f ms\n", c, ms); report += line;
-                if (ms < tbest) { tbest = ms; bestb = c; }
-            }
-            dp.add_blocks = bestb;
             if (tc_projector_supported(dp)) {
                 bool const before = dp.use_tc;
                 float t[2] = {0, 0};
@@ -120,18 +111,8 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
         }
         dp.local64_pencils = t[1] <= t[0];
     }
-    if (sizeof(T) == 8 && dp.nAI > 0 && dp.nCols > 0) {
-        float t[2] = {0, 0};
-        for (int v = 0; v < 2; ++v) {
-            dp.add64_unrolled = (1 == v);
-            if (!time_part<T>(dp, 1, y, x, ci, st, t[v])) return false;
-            std::snprintf(line, sizeof(line), "FP64 projector, addition %s: %.3f ms\n", v ? "unrolled" : "rolled", t[v]);
-            report += line;
-        }
-        dp.add64_unrolled = t[1] <= t[0];
-    }
-    std::snprintf(line, sizeof(line), "chosen: projector chunk %u, addition %u blocks per CTA, local %s, %s projector\n",
-                  dp.prj_chunk, dp.add_blocks, local_name[dp.local_variant],
+    std::snprintf(line, sizeof(line), "chosen: projector chunk %u, local %s, %s projector\n",
+                  dp.prj_chunk, local_name[dp.local_variant],
                   dp.use_tc ? "tensor-core" : "CUDA-core");
     report += line;
     A43G_CUDA_TRY(cudaStreamSynchronize(st));

@@ -43,6 +43,14 @@ constexpr uint32_t kMaxPrjItem = 40;           // positions per item at most
 // slot of a list position with its flags: last cube of its x-line, last line of its z-slab
 constexpr uint32_t kLineEnd = 1u << 30, kSlabEnd = 1u << 31, kSlotMask = kLineEnd - 1;
 
+// segment of the addition: up to kSegment cubes of one x-line of a source that have atom images
+// near, the points any image reaches, and the records [first, first + count) of the images
+constexpr uint32_t kSegment = 4, kNoSlot = 0xffffffffu;
+struct AddSegment { uint32_t blk[kSegment]; uint64_t any[kSegment]; uint32_t first, count, src, pad; };
+// one image near a segment: its first coefficient and basis size, and per cube of the segment the
+// slot (kNoSlot: not near) and the mask; the cubes share the y- and z-tables of yz_slot
+struct AddRecord { uint32_t coeff, lmax, slot[kSegment], yz_slot, pad; uint64_t mask[kSegment]; };
+
 struct DevicePlan {
     bool uploaded = false;       // plan geometry on the device
     bool values_dirty = true;    // potential / matrices / phases need re-upload
@@ -58,10 +66,8 @@ struct DevicePlan {
     uint32_t max_zline = 0;      // cubes in the longest z-line
     // schedule parameters, set by the autotuner (autotune.cu) or left at these defaults
     uint32_t prj_chunk = 0;          // blocks per projection work item (0: by the plan's size)
-    uint32_t add_blocks = 16;        // blocks per CTA of the FP32 addition
     int local_variant = 2;           // FP32: 0 rows with one-step-ahead loads, 1 plain rows, 2 pencils, 3 staged pencils
     bool local64_pencils = true;     // FP64: pencils with the planes on two threads, else the row kernel
-    bool add64_unrolled = true;      // FP64 addition: z-orders unrolled, else one at a time
     bool atom_chain3 = false;        // atom matrices by the collect/multiply/broadcast kernels instead of one
     uint32_t nlists[3] = {0, 0, 0};
 
@@ -82,7 +88,6 @@ struct DevicePlan {
     DeviceBuffer subset_dev;     // uint32 [nCols] diagonal block of each source column
     DeviceBuffer slot_H, slot_mask, prj_slot, add_slot;   // projector tables per (image, row)
     DeviceBuffer slot_H32;       // float copy of slot_H for the FP32 kernels
-    DeviceBuffer add_info;       // uint4 per SHOadd entry: slot, first coefficient of the image, basis size, 0
     int table_stride = 0;        // doubles per slot in slot_H
     DeviceBuffer dev_error;      // int: first error code recorded by a kernel (0: none)
     bool use_tc = true;          // FP32 projector on the tensor cores (else SIMT)
@@ -96,6 +101,8 @@ struct DevicePlan {
     struct PrjLine { uint32_t count = 0; size_t part_rows = 0; DeviceBuffer items, tickets; } prj_line;
     DeviceBuffer prj_rec, line_tab64, line_tab32;
     uint32_t nslots = 0;
+    uint32_t add_segments = 0;   // the addition along lines: AddSegment, AddRecord
+    DeviceBuffer add_seg, add_rec;
     DeviceBuffer prj_part;       // partial projection sums of multi-item groups
     // batch plans (GreenPlan::replicate): npairs (energy, k-point) pairs of nsrc_pair sources each
     uint32_t npairs = 1, nsrc_pair = 0;
@@ -117,7 +124,6 @@ struct DevicePlan {
 
 bool upload_plan(GreenPlan const &hp, DevicePlan &dp);
 // kernel attributes (dynamic shared memory above 48 KB) of the current device
-bool prepare_simt_kernels();
 bool prepare_local_kernels();
 bool prepare_tc_kernels();
 // kernel launch counter: n launches at once (replays of a captured graph)
@@ -167,15 +173,17 @@ bool tc_projector_supported(DevicePlan const &dp);
 bool launch_project_tc(DevicePlan &dp, float const *x, cudaStream_t st);
 bool launch_add_tc(DevicePlan &dp, float *y, uint16_t const *colIndex, cudaStream_t st);
 
-// sum-factorized projection and addition on the CUDA cores (projector_simt.cu, FP32 and FP64);
-// both stage blocks with 16-byte copies and need 16-byte aligned x and y
-bool simt_projector_supported(DevicePlan const &dp, void const *x, void const *y, size_t real_bytes);
-template <typename T> bool launch_project_simt(DevicePlan &dp, T const *x, cudaStream_t st);
+// projection and addition along lines of cubes on the CUDA cores (projector_line.cuh); x and y on
+// 16-byte boundaries (the kernels move 8 bytes per lane)
+inline bool line_projector_supported(void const *x, void const *y) {
+    return 0 == ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u);
+}
 // the projection along lines with the given tables (every coefficient of an active source is written)
 bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const *tab, cudaStream_t st);
 bool launch_project_line(DevicePlan &dp, double *apc, double const *x, void const *tab, cudaStream_t st);
+bool launch_add_line(DevicePlan &dp, float *y, float const *cad, cudaStream_t st);
+bool launch_add_line(DevicePlan &dp, double *y, double const *cad, cudaStream_t st);
 bool prepare_line_kernels32();
 bool prepare_line_kernels64();
-template <typename T> bool launch_add_simt(DevicePlan &dp, T *y, uint16_t const *colIndex, cudaStream_t st);
 
 } // namespace a43g

@@ -75,11 +75,12 @@ __global__ void k_line_table(double *t64, float2 *t32, double const *slot_H, siz
     if (t32) t32[k] = make_float2(float(h), float(h));
 }
 
+bool build_add_segments(GreenPlan const &hp, DevicePlan &dp);
+
 } // namespace
 
 bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
-    if (!prepare_simt_kernels() || !prepare_line_kernels32() || !prepare_line_kernels64() || !prepare_tc_kernels() ||
-        !prepare_local_kernels()) return false;
+    if (!prepare_line_kernels32() || !prepare_line_kernels64() || !prepare_tc_kernels() || !prepare_local_kernels()) return false;
     dp.nnzb = uint32_t(hp.nnzb()); dp.nRows = hp.nRows; dp.nCols = hp.nCols;
     dp.nAtoms = hp.nAtoms; dp.nAI = hp.nAtomImages;
     dp.ncoeffI = uint32_t(hp.ncoeff_images()); dp.ncoeffA = uint32_t(hp.ncoeff_atoms());
@@ -161,16 +162,7 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
                 }
         if (!put(dp.prj_rec, rec)) return false;
     }
-    {   // one 16-byte record per addition pair, so the kernel needs no dependent index loads
-        std::vector<uint32_t> info(4*size_t(hp.SHOadd.nnz()), 0u);
-        for (size_t k = 0; k < hp.SHOadd.nnz(); ++k) {
-            uint32_t const a = hp.SHOadd.col[k];
-            info[4*k + 0] = hp.add_slot[k];
-            info[4*k + 1] = hp.AtomImageStarts[a];
-            info[4*k + 2] = uint32_t(hp.AtomImageLmax[a]);
-        }
-        if (!put(dp.add_info, info)) return false;
-    }
+    if (!build_add_segments(hp, dp)) return false;
     if (!put(dp.subset_dev, hp.subset)) return false;
     {   // blocks of every source, in block order
         std::vector<uint32_t> start(hp.nCols + 1, 0), blocks(hp.nnzb());
@@ -200,9 +192,6 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
         // FP64 local kernel: "pencils" (default) or "rows"
         char const *l64 = std::getenv("A43G_LOCAL64");
         dp.local64_pencils = !(l64 && 0 == std::strcmp(l64, "rows"));
-        // FP64 addition: z-orders "unrolled" (default) or "rolled"
-        char const *a64 = std::getenv("A43G_ADD64");
-        dp.add64_unrolled = !(a64 && 0 == std::strcmp(a64, "rolled"));
         // atom-matrix chain: one kernel (default) or "three" (collect, multiply, broadcast)
         char const *ac = std::getenv("A43G_ATOM_CHAIN");
         dp.atom_chain3 = (ac && 0 == std::strcmp(ac, "three"));
@@ -258,6 +247,52 @@ bool build_prj_items(GreenPlan const &hp, DevicePlan &dp) {
     dp.prj_line.part_rows = rows;
     return put(dp.prj_line.items, line) && put(dp.prj_line.tickets, std::vector<uint32_t>(4*size_t(groups), 0u));
 }
+
+namespace {
+bool build_add_segments(GreenPlan const &hp, DevicePlan &dp) {
+    // numax 6 and 7 take segments of half the length (registers)
+    uint32_t const len = (dp.lmax_max <= 5) ? kSegment : kSegment/2;
+    std::vector<AddSegment> segs;
+    std::vector<AddRecord> recs;
+    recs.reserve(hp.SHOadd.nnz()/2 + 16);
+    auto close = [&](uint32_t const *blk, uint32_t n) {
+        AddSegment sg{};
+        sg.first = uint32_t(recs.size()); sg.src = hp.colindx[blk[0]];
+        uint32_t at[kSegment], end[kSegment];
+        for (uint32_t i = 0; i < n; ++i) { sg.blk[i] = blk[i]; at[i] = hp.SHOadd.start[blk[i]]; end[i] = hp.SHOadd.start[blk[i] + 1]; }
+        while (true) {                               // the images of the cubes, merged in ascending order
+            uint32_t a = kNoSlot;
+            for (uint32_t i = 0; i < n; ++i) if (at[i] < end[i]) a = std::min(a, hp.SHOadd.col[at[i]]);
+            if (kNoSlot == a) break;
+            AddRecord r{};
+            r.coeff = hp.AtomImageStarts[a]; r.lmax = uint32_t(hp.AtomImageLmax[a]);
+            for (uint32_t i = 0; i < kSegment; ++i) r.slot[i] = kNoSlot;
+            for (uint32_t i = 0; i < n; ++i) {
+                if (at[i] >= end[i] || hp.SHOadd.col[at[i]] != a) continue;
+                r.slot[i] = r.yz_slot = hp.add_slot[at[i]++];
+                r.mask[i] = hp.slot_mask[r.slot[i]];
+                sg.any[i] |= r.mask[i];
+            }
+            recs.push_back(r);
+        }
+        sg.count = uint32_t(recs.size()) - sg.first;
+        segs.push_back(sg);
+    };
+    auto const &K = hp.kinetic[0];
+    for (uint32_t il = 0; il < K.nlists(); ++il) {
+        uint32_t blk[kSegment], n = 0;
+        for (uint32_t k = K.start[il] + kNhalo; k < K.start[il + 1] && K.entry[k] > 0; ++k) {
+            uint32_t const b = uint32_t(K.entry[k] - 1);
+            if (hp.SHOadd.start[b] == hp.SHOadd.start[b + 1]) continue;
+            blk[n++] = b;
+            if (n == len) { close(blk, n); n = 0; }
+        }
+        if (n) close(blk, n);
+    }
+    dp.add_segments = uint32_t(segs.size());
+    return put(dp.add_seg, segs) && put(dp.add_rec, recs);
+}
+} // namespace
 
 bool make_line_table(DevicePlan const &dp, double const *slot_H, DeviceBuffer &t64, DeviceBuffer *t32, cudaStream_t st) {
     int const nu = dp.table_stride/12, lp = (dp.lmax_max | 1) + 1;

@@ -1,4 +1,4 @@
-// FP32 instantiations of the line-factorized projector (projector_line.cuh).
+// FP32 instantiations of the projector kernels along lines of cubes (projector_line.cuh).
 #include "projector_line.cuh"
 
 namespace a43g {
@@ -7,6 +7,10 @@ bool prepare_line_kernels32() { return line::prepare<float>(); }
 
 bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const *tab, cudaStream_t st) {
     return line::launch_project<float>(dp, apc, x, tab, st);
+}
+
+bool launch_add_line(DevicePlan &dp, float *y, float const *cad, cudaStream_t st) {
+    return line::launch_add<float>(dp, y, cad, dp.line_tab32.ptr, st);
 }
 
 } // namespace a43g

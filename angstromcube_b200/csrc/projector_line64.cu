@@ -1,4 +1,4 @@
-// FP64 instantiations of the line-factorized projector (projector_line.cuh).
+// FP64 instantiations of the projector kernels along lines of cubes (projector_line.cuh).
 #include "projector_line.cuh"
 
 namespace a43g {
@@ -7,6 +7,10 @@ bool prepare_line_kernels64() { return line::prepare<double>(); }
 
 bool launch_project_line(DevicePlan &dp, double *apc, double const *x, void const *tab, cudaStream_t st) {
     return line::launch_project<double>(dp, apc, x, tab, st);
+}
+
+bool launch_add_line(DevicePlan &dp, double *y, double const *cad, cudaStream_t st) {
+    return line::launch_add<double>(dp, y, cad, dp.line_tab64.ptr, st);
 }
 
 } // namespace a43g

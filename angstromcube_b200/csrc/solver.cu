@@ -1521,7 +1521,7 @@ int solve_batched(GreenPlan &hp, DevicePlan &dp, BatchCache &bc, a43g_solve_opti
         if (!err.empty()) { set_error(err); return A43G_ERR_ARGUMENT; }
         bc.dev.reset(new DevicePlan());
         bc.ws.reset(new SolverWorkspace());
-        bc.dev->prj_chunk = dp.prj_chunk; bc.dev->add_blocks = dp.add_blocks;
+        bc.dev->prj_chunk = dp.prj_chunk;
         if (!upload_plan(bc.host, *bc.dev)) return A43G_ERR_CUDA;
         bc.dev->local_variant = dp.local_variant; bc.dev->use_tc = dp.use_tc;
         bc.npairs = wave;
