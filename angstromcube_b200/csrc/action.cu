@@ -602,9 +602,11 @@ local_pencil_kernel(float *__restrict__ y, float const *__restrict__ x,
 // one z-plane: 16 consecutive columns of the real plane and the same columns of the imaginary
 // plane (two 128-byte segments per load).  The only couplings of the planes, -i Im(E) x and the
 // Bloch phases of halo cubes, take the partner plane's values by a warp shuffle (lane ^ 16).
-// Registers hold the same number of values as the FP32 kernel's, at twice the bytes.
+// Registers hold the same number of values as the FP32 kernel's, at twice the bytes.  Measured on
+// the 64-atom cell with 8 sources (4.3 GB read and written once): 2.37 ms with 32-byte rows in shared
+// memory, whose 16-byte accesses met in the same banks twice, 1.80 ms with their halves apart.
 constexpr int kPencil64S = 16;
-constexpr int kPencil64Smem = 3*2*16*kPencil64S*32;   // bytes of the three z-slots (double4 rows)
+constexpr int kPencil64Smem = 3*2*16*kPencil64S*32;   // bytes of the three z-slots (rows of 4 doubles)
 
 struct Quad64 { double v[16]; };                     // one plane of [y*4 + x] of one z-plane of a cube
 
@@ -633,7 +635,7 @@ local_pencil64_kernel(double *__restrict__ y, double const *__restrict__ x,
                       double const *__restrict__ Vcell, LocalArgs<double> a)
 {
     constexpr int S = kPencil64S, NSL = 64/S;
-    extern __shared__ __align__(16) double4 slot64[];  // [3][2][16][S]
+    extern __shared__ __align__(16) double2 slot64[];  // [3][2][16][2 halves of a row][S]
     __shared__ int32_t code[kMaxLine][8];              // per step: block, x-, x+, y-, y+, veff, z-next
     __shared__ int32_t zleft, nline;
     int const line = blockIdx.x/NSL, slice = blockIdx.x % NSL;
@@ -654,11 +656,17 @@ local_pencil64_kernel(double *__restrict__ y, double const *__restrict__ x,
         code[k][0] = b; code[k][1] = nb[0]; code[k][2] = nb[1]; code[k][3] = nb[2]; code[k][4] = nb[3];
         code[k][5] = veff[b]; code[k][6] = list_code(L[5 + k]);
     }
-    auto srow = [&](int slot, int plane, int row) -> double4 & { return slot64[((slot*2 + plane)*16 + row)*S + j]; };
+    // the halves of a row are S apart, so that the 16-byte accesses of a quarter warp are contiguous
+    // (whole rows of 32 bytes per lane met in the same banks twice)
+    auto srow = [&](int slot, int plane, int row, int half) -> double2 & {
+        return slot64[(((slot*2 + plane)*16 + row)*2 + half)*S + j];
+    };
     auto put = [&](int slot, Quad64 const &q) {
 #pragma unroll
         for (int yy = 0; yy < 4; ++yy)
-            srow(slot, pl, zq*4 + yy) = make_double4(q.v[yy*4], q.v[yy*4 + 1], q.v[yy*4 + 2], q.v[yy*4 + 3]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                srow(slot, pl, zq*4 + yy, h) = make_double2(q.v[yy*4 + 2*h], q.v[yy*4 + 2*h + 1]);
     };
     auto qphase = [&](int32_t e, double pr, double pi, Quad64 &q) {
         if (e < -1) {
@@ -693,8 +701,8 @@ local_pencil64_kernel(double *__restrict__ y, double const *__restrict__ x,
         double cur[16];
 #pragma unroll
         for (int yy = 0; yy < 4; ++yy) {
-            double4 const v = srow(sc, pl, zq*4 + yy);
-            cur[yy*4] = v.x; cur[yy*4 + 1] = v.y; cur[yy*4 + 2] = v.z; cur[yy*4 + 3] = v.w;
+            double2 const v = srow(sc, pl, zq*4 + yy, 0), u = srow(sc, pl, zq*4 + yy, 1);
+            cur[yy*4] = v.x; cur[yy*4 + 1] = v.y; cur[yy*4 + 2] = u.x; cur[yy*4 + 3] = u.y;
         }
         double acc[16];
         // potential and centre; the other plane of the own points from the partner lane
@@ -778,11 +786,12 @@ local_pencil64_kernel(double *__restrict__ y, double const *__restrict__ x,
                 int const zm = zq - d, zp = zq + d;
                 int const s_m = (zm < 0) ? sp : sc, s_p = (zp > 3) ? sn : sc;
                 int const r_m = (zm & 3)*4 + yy, r_p = (zp & 3)*4 + yy;
-                double4 const m = srow(s_m, pl, r_m), p = srow(s_p, pl, r_p);
-                acc[yy*4 + 0] += cz[d]*(m.x + p.x);
-                acc[yy*4 + 1] += cz[d]*(m.y + p.y);
-                acc[yy*4 + 2] += cz[d]*(m.z + p.z);
-                acc[yy*4 + 3] += cz[d]*(m.w + p.w);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    double2 const m = srow(s_m, pl, r_m, h), p = srow(s_p, pl, r_p, h);
+                    acc[yy*4 + 2*h] += cz[d]*(m.x + p.x);
+                    acc[yy*4 + 2*h + 1] += cz[d]*(m.y + p.y);
+                }
             }
         double *yb = y + size_t(b)*kBlockReals + pl*4096 + (zq*16)*64 + col;
 #pragma unroll
