@@ -10,6 +10,7 @@
 //    (include/green_dyadic.hxx:856-922), with the image/atom coefficient scratch owned by
 //    the plan instead of being allocated on every call.
 #include "device.cuh"
+#include "lane8.cuh"
 
 #include <algorithm>
 
@@ -237,779 +238,179 @@ local_fused_kernel(T *__restrict__ y, T const *__restrict__ x,
     }
 }
 
-// The same fused local operator with the global loads of every step issued one step ahead:
-// the neighbour codes of the whole z-line are read into shared memory once, so the rows of cube
-// k+1 (its z-successor, its y and x neighbours and its potential row) are requested before cube
-// k is computed and arrive while it is.  Bloch phases are applied when the rows are consumed.
-// Lines of at most kMaxLine cubes (the host checks).
-constexpr int kMaxLine = 128;
-
-template <typename T> struct Rows { T re[4], im[4]; };
+// Pencil kernel (FP32 and FP64): one CTA per (z-line, group of 16 lanes of columns).  A lane holds 8
+// bytes of columns, one in FP64, two in FP32 (.f32x2 arithmetic); a warp is one z-plane zq, its two
+// halves the planes re and im.  A thread owns the 16 points of its plane: the x- and y-stencils run
+// in registers, the rows of the x- and y-neighbours come straight from global memory (the L2) and
+// are applied as they arrive.  Only the z-stencil reads shared memory, where the previous, current
+// and next cube of the line are staged by 16-byte asynchronous copies, [slot][re, im][point][lane]
+// (a half warp reads 128 contiguous bytes); the copy of the cube after the next one starts as soon
+// as the z-stencil is done with the previous cube.  The only couplings of re and im, -i Im(E) x and
+// the Bloch phases of halo cubes, take the other plane's values from the partner lane (lane ^ 16).
+//
+// Measured on the 64-atom cell with 8 sources (32,768 blocks): FP64 1.61 ms (4.3 GB read and written
+// once: 0.66 ms), FP32 0.83 ms.  With the z-successor held in registers a step ahead instead of
+// copied, one FP32 column per lane, and the length of the line found by walking it: 1.80 and 0.89
+// ms.  Three CTAs per SM in FP64 (168 registers) rather than four: at 128 registers too few of the
+// neighbour rows' loads are in flight (1.92 ms).  What bounds it: the latency of those loads, and
+// the 8 shared-memory reads per point of the z-stencil.
+constexpr int kMaxLine = 128;        // cubes of a line (the host checks)
+constexpr int kPencilThreads = 128;
+constexpr int kPencilSmem = 3*2*64*16*8;          // bytes of the three z-slots
 
 template <typename T>
-__device__ __forceinline__ void row_raw(T const *__restrict__ x, int32_t e, int r, int col, Rows<T> &o) {
-    if (-1 == e) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { o.re[i] = T(0); o.im[i] = T(0); }
-        return;
-    }
-    T const *b = x + size_t(nbr_block(e))*kBlockReals + (r*4)*64 + col;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { o.re[i] = __ldg(b + i*64); o.im[i] = __ldg(b + 4096 + i*64); }
-}
-
-template <typename T>
-__device__ __forceinline__ void row_phase(int32_t e, T pr, T pi, Rows<T> &o) {
-    if (e < -1) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            T const a = pr*o.re[i] - pi*o.im[i], c = pr*o.im[i] + pi*o.re[i];
-            o.re[i] = a; o.im[i] = c;
-        }
-    }
-}
-
-template <typename T, int S>
-__global__ void __launch_bounds__(S*16, 2)
-local_fused_pf_kernel(T *__restrict__ y, T const *__restrict__ x,
-                      uint32_t const *__restrict__ zstart, int32_t const *__restrict__ zlist,
-                      int32_t const *__restrict__ nbr, int32_t const *__restrict__ veff,
-                      T const *__restrict__ Vcell, LocalArgs<T> a)
-{
-    constexpr int NSL = 64/S, PAD = 68;
-    __shared__ __align__(16) T sm[5][2][S][PAD];   // slots: 3 rotating z-slots, y-, y+
-    __shared__ int32_t code[kMaxLine][8];           // per step: block, x-, x+, y-, y+, veff, z-next
-    __shared__ int32_t zleft, nline;
-    int const line = blockIdx.x/NSL, slice = blockIdx.x % NSL;
-    int const tid = threadIdx.x, j = tid % S, r = tid/S;       // r = z*4 + y
-    int const zq = r >> 2, yq = r & 3, col = slice*S + j;
-    int32_t const *L = zlist + zstart[line];
-    if (0 == tid) {
-        int n = 0;
-        while (L[4 + n] > 0) ++n;                   // lists end with 4 non-positive entries
-        nline = n; zleft = list_code(L[3]);
-    }
-    __syncthreads();
-    int const n = nline;
-    if (0 == n || !line_args(a, L[4] - 1)) return;  // uniform: nothing on this line, or retired
-    for (int k = tid; k < n; k += S*16) {
-        int32_t const b = L[4 + k] - 1;
-        int32_t const *nb = nbr + 6*size_t(b);
-        code[k][0] = b; code[k][1] = nb[0]; code[k][2] = nb[1]; code[k][3] = nb[2]; code[k][4] = nb[3];
-        code[k][5] = veff[b]; code[k][6] = list_code(L[5 + k]);
-    }
-    __syncthreads();
-    T const (&cx)[5] = a.st.c[0];
-    T const (&cy)[5] = a.st.c[1];
-    T const (&cz)[5] = a.st.c[2];
-    T const c0 = cx[0] + cy[0] + cz[0];
-
-    Rows<T> cur;                                     // own row of the current cube
-    {
-        Rows<T> h;
-        row_raw(x, zleft, r, col, h);
-        row_phase(zleft, a.ph[2][0][0], a.ph[2][0][1], h);
-        sts_row(&sm[0][0][j][r*4], h.re); sts_row(&sm[0][1][j][r*4], h.im);
-    }
-    row_raw(x, code[0][0], r, col, cur);
-    sts_row(&sm[1][0][j][r*4], cur.re); sts_row(&sm[1][1][j][r*4], cur.im);
-    // rows of step 0 requested before the loop
-    Rows<T> pz, pym, pyp, pxm, pxp;
-    Row4<T> pV;
-    auto request = [&](int k) {
-        row_raw(x, code[k][6], r, col, pz);
-        row_raw(x, code[k][3], r, col, pym);
-        row_raw(x, code[k][4], r, col, pyp);
-        row_raw(x, code[k][1], r, col, pxm);
-        row_raw(x, code[k][2], r, col, pxp);
-        int32_t const iloc = code[k][5];
-        if (iloc < 0) { pV.v[0] = pV.v[1] = pV.v[2] = pV.v[3] = T(0); }
-        else pV = lds_row_global(Vcell + size_t(iloc)*64 + r*4);
-    };
-    request(0);
-    int sp = 0, sc = 1, sn = 2;
-    for (int k = 0; k < n; ++k) {
-        int32_t const b = code[k][0];
-        row_phase(code[k][6], a.ph[2][1][0], a.ph[2][1][1], pz);
-        row_phase(code[k][3], a.ph[1][0][0], a.ph[1][0][1], pym);
-        row_phase(code[k][4], a.ph[1][1][0], a.ph[1][1][1], pyp);
-        row_phase(code[k][1], a.ph[0][0][0], a.ph[0][0][1], pxm);
-        row_phase(code[k][2], a.ph[0][1][0], a.ph[0][1][1], pxp);
-        __syncthreads();                             // previous step finished reading the slots
-        sts_row(&sm[sn][0][j][r*4], pz.re);  sts_row(&sm[sn][1][j][r*4], pz.im);
-        sts_row(&sm[3][0][j][r*4], pym.re);  sts_row(&sm[3][1][j][r*4], pym.im);
-        sts_row(&sm[4][0][j][r*4], pyp.re);  sts_row(&sm[4][1][j][r*4], pyp.im);
-        __syncthreads();
-        T lr[12], li[12];                            // x-line: left row | own row | right row
-        T V[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            lr[i] = pxm.re[i]; li[i] = pxm.im[i];
-            lr[4 + i] = cur.re[i]; li[4 + i] = cur.im[i];
-            lr[8 + i] = pxp.re[i]; li[8 + i] = pxp.im[i];
-            V[i] = pV.v[i];
-        }
-        Rows<T> const nextc = pz;
-        if (k + 1 < n) request(k + 1);               // arrives while this cube is computed
-        T accr[4], acci[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            T const Vt = V[i] - a.E_re;
-            accr[i] = Vt*cur.re[i] + a.E_im*cur.im[i] + c0*cur.re[i];
-            acci[i] = Vt*cur.im[i] - a.E_im*cur.re[i] + c0*cur.im[i];
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int d = 1; d <= 4; ++d) {
-                accr[i] += cx[d]*(lr[4 + i - d] + lr[4 + i + d]);
-                acci[i] += cx[d]*(li[4 + i - d] + li[4 + i + d]);
-            }
-#pragma unroll
-        for (int d = 1; d <= 4; ++d) {
-            int const ym = yq - d, yp = yq + d, zm = zq - d, zp = zq + d;
-            int const s_ym = (ym < 0) ? 3 : sc, s_yp = (yp > 3) ? 4 : sc;
-            int const s_zm = (zm < 0) ? sp : sc, s_zp = (zp > 3) ? sn : sc;
-            int const o_ym = (zq*4 + (ym & 3))*4, o_yp = (zq*4 + (yp & 3))*4;
-            int const o_zm = ((zm & 3)*4 + yq)*4, o_zp = ((zp & 3)*4 + yq)*4;
-            Row4<T> const r1 = lds_row(&sm[s_ym][0][j][o_ym]), r2 = lds_row(&sm[s_yp][0][j][o_yp]);
-            Row4<T> const r3 = lds_row(&sm[s_zm][0][j][o_zm]), r4 = lds_row(&sm[s_zp][0][j][o_zp]);
-            Row4<T> const i1 = lds_row(&sm[s_ym][1][j][o_ym]), i2 = lds_row(&sm[s_yp][1][j][o_yp]);
-            Row4<T> const i3 = lds_row(&sm[s_zm][1][j][o_zm]), i4 = lds_row(&sm[s_zp][1][j][o_zp]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                accr[i] += cy[d]*(r1.v[i] + r2.v[i]) + cz[d]*(r3.v[i] + r4.v[i]);
-                acci[i] += cy[d]*(i1.v[i] + i2.v[i]) + cz[d]*(i3.v[i] + i4.v[i]);
-            }
-        }
-        T *yb = y + size_t(b)*kBlockReals + (r*4)*64 + col;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { yb[i*64] = accr[i]; yb[4096 + i*64] = acci[i]; }
-        int const t = sp; sp = sc; sc = sn; sn = t;  // rotate the z-slots
-        cur = nextc;
-    }
-}
-
-// Pencil variant (FP32): one CTA per (z-line, slice of S = 32 columns); thread (zq, j) owns the
-// four y-rows (zq, y = 0..3) of every cube of the line for column j, so one warp covers 32
-// consecutive columns of one z-plane (128-byte loads and stores).  The x- and y-stencils run in
-// registers: the x- and y-neighbour rows come straight from global memory (the L2) and are
-// applied in scatter form as they arrive.  Only the z-stencil reads shared memory, where the
-// previous, current and next cube of the line are staged as 16-byte rows, [slot][plane][row][S]
-// (a quarter warp reads 128 contiguous bytes: no bank conflicts).  Per output point this reads
-// half the shared-memory bytes of the row kernel above and passes a barrier a quarter as often.
-// The z-successor of the next cube is requested one step ahead.
-constexpr int kPencilS = 32;
-constexpr int kPencilSmem = 3*2*16*kPencilS*16;   // bytes of the three z-slots
-
-struct Quad { float v[2][16]; };                 // [plane][y*4 + x] of one z-plane of a cube
-
-__device__ __forceinline__ void quad_raw(float const *__restrict__ x, int32_t e, int zq, int col, Quad &q) {
-    if (-1 == e) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { q.v[0][i] = 0.f; q.v[1][i] = 0.f; }
-        return;
-    }
-    float const *b = x + size_t(nbr_block(e))*kBlockReals + (zq*16)*64 + col;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) { q.v[0][i] = __ldg(b + i*64); q.v[1][i] = __ldg(b + 4096 + i*64); }
-}
-
-__device__ __forceinline__ void quad_phase(int32_t e, float pr, float pi, Quad &q) {
-    if (e < -1) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float const a = pr*q.v[0][i] - pi*q.v[1][i], c = pr*q.v[1][i] + pi*q.v[0][i];
-            q.v[0][i] = a; q.v[1][i] = c;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(4*kPencilS, 4)
-local_pencil_kernel(float *__restrict__ y, float const *__restrict__ x,
+__global__ void __launch_bounds__(kPencilThreads, sizeof(T) == 8 ? 3 : 4)
+local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
                     uint32_t const *__restrict__ zstart, int32_t const *__restrict__ zlist,
                     int32_t const *__restrict__ nbr, int32_t const *__restrict__ veff,
-                    float const *__restrict__ Vcell, LocalArgs<float> a)
+                    T const *__restrict__ Vcell, T const *__restrict__ zero, LocalArgs<T> a)
 {
-    constexpr int S = kPencilS, NSL = 64/S;
-    extern __shared__ __align__(16) float4 slot4[];   // [3][2][16][S]
+    using V = typename LaneOf<T>::V;
+    constexpr int W = 8/int(sizeof(T)), S = 64/W, NG = S/16;   // columns per lane, lanes per point, groups
+    extern __shared__ __align__(16) unsigned char slot_raw[];
+    V *slots = reinterpret_cast<V*>(slot_raw);         // [3][2][64][16]
     __shared__ int32_t code[kMaxLine][8];              // per step: block, x-, x+, y-, y+, veff, z-next
-    __shared__ int32_t zleft, nline;
-    int const line = blockIdx.x/NSL, slice = blockIdx.x % NSL;
-    int const tid = threadIdx.x, j = tid % S, zq = tid/S, col = slice*S + j;
+    int const line = blockIdx.x/NG, group = blockIdx.x % NG;
+    int const tid = threadIdx.x, lane = tid & 31, zq = tid >> 5, pl = lane >> 4, j = lane & 15;
     int32_t const *L = zlist + zstart[line];
-    if (0 == tid) {
-        int n = 0;
-        while (L[4 + n] > 0) ++n;                   // lists end with 4 non-positive entries
-        nline = n; zleft = list_code(L[3]);
-    }
-    __syncthreads();
-    int const n = nline;
-    if (0 == n || !line_args(a, L[4] - 1)) return;  // uniform: nothing on this line, or retired
-    for (int k = tid; k < n; k += 4*S) {
+    int const n = int(zstart[line + 1] - zstart[line]) - 8;    // lists have 4 halo entries at both ends
+    if (n < 1 || !line_args(a, L[4] - 1)) return;      // uniform: nothing on this line, or retired
+    int32_t const zleft = list_code(L[3]);
+    for (int k = tid; k < n; k += kPencilThreads) {
         int32_t const b = L[4 + k] - 1;
         int32_t const *nb = nbr + 6*size_t(b);
         code[k][0] = b; code[k][1] = nb[0]; code[k][2] = nb[1]; code[k][3] = nb[2]; code[k][4] = nb[3];
         code[k][5] = veff[b]; code[k][6] = list_code(L[5 + k]);
     }
-    auto srow = [&](int slot, int pl, int row) -> float4 & { return slot4[((slot*2 + pl)*16 + row)*S + j]; };
-    auto put = [&](int slot, Quad const &q) {
+    size_t const lo = size_t(pl)*4096 + group*16*W + j*W;      // element of this lane at point 0
+    V *mine = slots + (pl*64 + zq*16)*16 + j;                  // this thread's points of slot 0
+    constexpr int SLOT = 2*64*16;
+    auto fetch = [&](int slot, int32_t e) {                    // cube e into a slot (-1: zeros)
+        V *dst = slots + slot*SLOT;
+        if (-1 == e) {
 #pragma unroll
-        for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-            for (int pl = 0; pl < 2; ++pl)
-                srow(slot, pl, zq*4 + yy) = make_float4(q.v[pl][yy*4], q.v[pl][yy*4 + 1], q.v[pl][yy*4 + 2], q.v[pl][yy*4 + 3]);
-    };
-    float const (&cx)[5] = a.st.c[0];
-    float const (&cy)[5] = a.st.c[1];
-    float const (&cz)[5] = a.st.c[2];
-    float const c0 = cx[0] + cy[0] + cz[0];
-    __syncthreads();                                // code[] complete
-    {
-        Quad h;
-        quad_raw(x, zleft, zq, col, h);
-        quad_phase(zleft, a.ph[2][0][0], a.ph[2][0][1], h);
-        put(0, h);
-        quad_raw(x, code[0][0], zq, col, h);
-        put(1, h);
-    }
-    Quad nx;                                        // rows of the z-successor, one step ahead
-    quad_raw(x, code[0][6], zq, col, nx);
-    int sp = 0, sc = 1, sn = 2;
-    for (int k = 0; k < n; ++k) {
-        int32_t const b = code[k][0];
-        quad_phase(code[k][6], a.ph[2][1][0], a.ph[2][1][1], nx);   // only the line end has a phase
-        __syncthreads();                            // the previous step finished reading slot sn
-        put(sn, nx);
-        __syncthreads();
-        if (k + 1 < n) quad_raw(x, code[k + 1][6], zq, col, nx);   // arrives during this step
-        Quad cur;
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-            for (int pl = 0; pl < 2; ++pl) {
-                float4 const v = srow(sc, pl, zq*4 + yy);
-                cur.v[pl][yy*4] = v.x; cur.v[pl][yy*4 + 1] = v.y; cur.v[pl][yy*4 + 2] = v.z; cur.v[pl][yy*4 + 3] = v.w;
-            }
-        float acc[2][16];
-        // potential and centre
-        int32_t const iloc = code[k][5];
-        float V[16];
-        if (iloc < 0) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) V[i] = 0.f;
+            for (int i = 0; i < 16; ++i) mine[slot*SLOT + i*16] = V(0);
         } else {
+            T const *src = x + size_t(nbr_block(e))*kBlockReals + group*16*W;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float4 const v = __ldg(reinterpret_cast<float4 const*>(Vcell + size_t(iloc)*64 + zq*16 + q*4));
-                V[q*4] = v.x; V[q*4 + 1] = v.y; V[q*4 + 2] = v.z; V[q*4 + 3] = v.w;
+            for (int q = 0; q < 2*64*8/kPencilThreads; ++q) {
+                int const c = q*kPencilThreads + tid, row = c >> 3, part = c & 7;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::
+                             "r"(uint32_t(__cvta_generic_to_shared(dst + row*16 + 2*part))), "l"(src + row*64 + part*2*W) : "memory");
             }
         }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float const Vt = V[i] - a.E_re;
-            acc[0][i] = Vt*cur.v[0][i] + a.E_im*cur.v[1][i] + c0*cur.v[0][i];
-            acc[1][i] = Vt*cur.v[1][i] - a.E_im*cur.v[0][i] + c0*cur.v[1][i];
-        }
-        // y-stencil inside the cube
-#pragma unroll
-        for (int pl = 0; pl < 2; ++pl)
-#pragma unroll
-            for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-                for (int yo = 0; yo < 4; ++yo) {
-                    if (yo == yy) continue;
-                    int const d = (yo > yy) ? yo - yy : yy - yo;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[pl][yy*4 + i] += cy[d]*cur.v[pl][yo*4 + i];
-                }
-        // x-stencil: the rows of the x-neighbours at (zq, yy)
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy) {
-            Rows<float> xm, xp;
-            row_raw(x, code[k][1], zq*4 + yy, col, xm);
-            row_raw(x, code[k][2], zq*4 + yy, col, xp);
-            row_phase(code[k][1], a.ph[0][0][0], a.ph[0][0][1], xm);
-            row_phase(code[k][2], a.ph[0][1][0], a.ph[0][1][1], xp);
-            float lr[12], li[12];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                lr[i] = xm.re[i]; li[i] = xm.im[i];
-                lr[4 + i] = cur.v[0][yy*4 + i]; li[4 + i] = cur.v[1][yy*4 + i];
-                lr[8 + i] = xp.re[i]; li[8 + i] = xp.im[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int d = 1; d <= 4; ++d) {
-                    acc[0][yy*4 + i] += cx[d]*(lr[4 + i - d] + lr[4 + i + d]);
-                    acc[1][yy*4 + i] += cx[d]*(li[4 + i - d] + li[4 + i + d]);
-                }
-        }
-        // y-neighbour cubes: row yo of y- sits at y = yo - 4, row yo of y+ at y = yo + 4
-#pragma unroll
-        for (int yo = 0; yo < 4; ++yo) {
-            Rows<float> ym, yp;
-            row_raw(x, code[k][3], zq*4 + yo, col, ym);
-            row_raw(x, code[k][4], zq*4 + yo, col, yp);
-            row_phase(code[k][3], a.ph[1][0][0], a.ph[1][0][1], ym);
-            row_phase(code[k][4], a.ph[1][1][0], a.ph[1][1][1], yp);
-#pragma unroll
-            for (int yy = 0; yy < 4; ++yy) {
-                if (yy <= yo) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        acc[0][yy*4 + i] += cy[yy - yo + 4]*ym.re[i];
-                        acc[1][yy*4 + i] += cy[yy - yo + 4]*ym.im[i];
-                    }
-                }
-                if (yy >= yo) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        acc[0][yy*4 + i] += cy[yo + 4 - yy]*yp.re[i];
-                        acc[1][yy*4 + i] += cy[yo + 4 - yy]*yp.im[i];
-                    }
-                }
-            }
-        }
-        // z-stencil from the three staged cubes (previous, current, next)
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-            for (int d = 1; d <= 4; ++d) {
-                int const zm = zq - d, zp = zq + d;
-                int const s_m = (zm < 0) ? sp : sc, s_p = (zp > 3) ? sn : sc;
-                int const r_m = (zm & 3)*4 + yy, r_p = (zp & 3)*4 + yy;
-#pragma unroll
-                for (int pl = 0; pl < 2; ++pl) {
-                    float4 const m = srow(s_m, pl, r_m), p = srow(s_p, pl, r_p);
-                    acc[pl][yy*4 + 0] += cz[d]*(m.x + p.x);
-                    acc[pl][yy*4 + 1] += cz[d]*(m.y + p.y);
-                    acc[pl][yy*4 + 2] += cz[d]*(m.z + p.z);
-                    acc[pl][yy*4 + 3] += cz[d]*(m.w + p.w);
-                }
-            }
-        float *yb = y + size_t(b)*kBlockReals + (zq*16)*64 + col;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { yb[i*64] = acc[0][i]; yb[4096 + i*64] = acc[1][i]; }
-        int const t = sp; sp = sc; sc = sn; sn = t;  // rotate the z-slots
-    }
-}
-
-// Pencil variant in FP64: the pencil kernel's mapping with the two planes on two threads.  One
-// CTA of 128 threads per (z-line, slice of 16 columns); thread (zq, plane, j) owns one plane (re
-// or im) of the four y-rows (zq, y = 0..3) of every cube of the line for column j, so a warp is
-// one z-plane: 16 consecutive columns of the real plane and the same columns of the imaginary
-// plane (two 128-byte segments per load).  The only couplings of the planes, -i Im(E) x and the
-// Bloch phases of halo cubes, take the partner plane's values by a warp shuffle (lane ^ 16).
-// Registers hold the same number of values as the FP32 kernel's, at twice the bytes.  Measured on
-// the 64-atom cell with 8 sources (4.3 GB read and written once): 2.37 ms with 32-byte rows in shared
-// memory, whose 16-byte accesses met in the same banks twice, 1.80 ms with their halves apart.
-constexpr int kPencil64S = 16;
-constexpr int kPencil64Smem = 3*2*16*kPencil64S*32;   // bytes of the three z-slots (rows of 4 doubles)
-
-struct Quad64 { double v[16]; };                     // one plane of [y*4 + x] of one z-plane of a cube
-
-__device__ __forceinline__ void quad64_raw(double const *__restrict__ x, int32_t e, int zq, int pl, int col, Quad64 &q) {
-    if (-1 == e) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) q.v[i] = 0.0;
-        return;
-    }
-    double const *b = x + size_t(nbr_block(e))*kBlockReals + pl*4096 + (zq*16)*64 + col;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) q.v[i] = __ldg(b + i*64);
-}
-
-// rotation by the Bloch phase (pr, pi) of a halo cube, uniform over the CTA: re' = pr re - pi im,
-// im' = pr im + pi re, with the other plane from the partner lane
-__device__ __forceinline__ double phase64(double v, int pl, double pr, double pi) {
-    double const w = __shfl_xor_sync(0xffffffffu, v, 16);
-    return pr*v + (pl ? pi : -pi)*w;
-}
-
-__global__ void __launch_bounds__(8*kPencil64S, 3)
-local_pencil64_kernel(double *__restrict__ y, double const *__restrict__ x,
-                      uint32_t const *__restrict__ zstart, int32_t const *__restrict__ zlist,
-                      int32_t const *__restrict__ nbr, int32_t const *__restrict__ veff,
-                      double const *__restrict__ Vcell, LocalArgs<double> a)
-{
-    constexpr int S = kPencil64S, NSL = 64/S;
-    extern __shared__ __align__(16) double2 slot64[];  // [3][2][16][2 halves of a row][S]
-    __shared__ int32_t code[kMaxLine][8];              // per step: block, x-, x+, y-, y+, veff, z-next
-    __shared__ int32_t zleft, nline;
-    int const line = blockIdx.x/NSL, slice = blockIdx.x % NSL;
-    int const tid = threadIdx.x, lane = tid & 31, zq = tid >> 5;
-    int const pl = lane >> 4, j = lane & 15, col = slice*S + j;
-    int32_t const *L = zlist + zstart[line];
-    if (0 == tid) {
-        int n = 0;
-        while (L[4 + n] > 0) ++n;                   // lists end with 4 non-positive entries
-        nline = n; zleft = list_code(L[3]);
-    }
-    __syncthreads();
-    int const n = nline;
-    if (0 == n || !line_args(a, L[4] - 1)) return;  // uniform: nothing on this line, or retired
-    for (int k = tid; k < n; k += 8*S) {
-        int32_t const b = L[4 + k] - 1;
-        int32_t const *nb = nbr + 6*size_t(b);
-        code[k][0] = b; code[k][1] = nb[0]; code[k][2] = nb[1]; code[k][3] = nb[2]; code[k][4] = nb[3];
-        code[k][5] = veff[b]; code[k][6] = list_code(L[5 + k]);
-    }
-    // the halves of a row are S apart, so that the 16-byte accesses of a quarter warp are contiguous
-    // (whole rows of 32 bytes per lane met in the same banks twice)
-    auto srow = [&](int slot, int plane, int row, int half) -> double2 & {
-        return slot64[(((slot*2 + plane)*16 + row)*2 + half)*S + j];
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto put = [&](int slot, Quad64 const &q) {
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                srow(slot, pl, zq*4 + yy, h) = make_double2(q.v[yy*4 + 2*h], q.v[yy*4 + 2*h + 1]);
+    auto land = [&]() {                                        // all copies, everybody's
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
     };
-    auto qphase = [&](int32_t e, double pr, double pi, Quad64 &q) {
-        if (e < -1) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) q.v[i] = phase64(q.v[i], pl, pr, pi);
-        }
+    auto phase = [&](V v, T pr, T pi) {
+        return vfma(vdup(pr), v, vmul(vdup(pl ? pi : -pi), __shfl_xor_sync(0xffffffffu, v, 16)));
     };
-    double const (&cx)[5] = a.st.c[0];
-    double const (&cy)[5] = a.st.c[1];
-    double const (&cz)[5] = a.st.c[2];
-    double const c0 = cx[0] + cy[0] + cz[0];
-    double const Eim = pl ? -a.E_im : a.E_im;       // re: + Im(E) im, im: - Im(E) re
-    __syncthreads();                                // code[] complete
-    {
-        Quad64 h;
-        quad64_raw(x, zleft, zq, pl, col, h);
-        qphase(zleft, a.ph[2][0][0], a.ph[2][0][1], h);
-        put(0, h);
-        quad64_raw(x, code[0][0], zq, pl, col, h);
-        put(1, h);
-    }
-    Quad64 nx;                                      // rows of the z-successor, one step ahead
-    quad64_raw(x, code[0][6], zq, pl, col, nx);
+    auto turn = [&](int slot, T const (&ph)[2]) {              // Bloch phase of a staged halo cube
+#pragma unroll
+        for (int i = 0; i < 16; ++i) mine[slot*SLOT + i*16] = phase(mine[slot*SLOT + i*16], ph[0], ph[1]);
+    };
+    auto base = [&](int32_t e) {                               // this thread's plane of neighbour e
+        T const *p = (-1 == e) ? zero : x + size_t(nbr_block(e))*kBlockReals;
+        return reinterpret_cast<V const*>(p + lo) + zq*16*S;
+    };
+    V const cx1 = vdup(a.st.c[0][1]), cx2 = vdup(a.st.c[0][2]), cx3 = vdup(a.st.c[0][3]), cx4 = vdup(a.st.c[0][4]);
+    V const cy1 = vdup(a.st.c[1][1]), cy2 = vdup(a.st.c[1][2]), cy3 = vdup(a.st.c[1][3]), cy4 = vdup(a.st.c[1][4]);
+    V const cz1 = vdup(a.st.c[2][1]), cz2 = vdup(a.st.c[2][2]), cz3 = vdup(a.st.c[2][3]), cz4 = vdup(a.st.c[2][4]);
+    V const cx[5] = {V(0), cx1, cx2, cx3, cx4}, cy[5] = {V(0), cy1, cy2, cy3, cy4}, cz[5] = {V(0), cz1, cz2, cz3, cz4};
+    T const shift = (a.st.c[0][0] + a.st.c[1][0] + a.st.c[2][0]) - a.E_re;
+    V const eim = vdup(pl ? -a.E_im : a.E_im);                 // re: + Im(E) im, im: - Im(E) re
+    __syncthreads();                                           // code[] complete
+    fetch(0, zleft); fetch(1, code[0][0]); fetch(2, code[0][6]);
+    land();
+    if (zleft < -1) turn(0, a.ph[2][0]);
+    if (code[0][6] < -1) turn(2, a.ph[2][1]);
+    if (zleft < -1 || code[0][6] < -1) __syncthreads();
     int sp = 0, sc = 1, sn = 2;
     for (int k = 0; k < n; ++k) {
-        int32_t const b = code[k][0];
-        qphase(code[k][6], a.ph[2][1][0], a.ph[2][1][1], nx);       // only the line end has a phase
-        __syncthreads();                            // the previous step finished reading slot sn
-        put(sn, nx);
-        __syncthreads();
-        if (k + 1 < n) quad64_raw(x, code[k + 1][6], zq, pl, col, nx);   // arrives during this step
-        double cur[16];
+        int32_t const exm = code[k][1], exp_ = code[k][2], eym = code[k][3], eyp = code[k][4], iloc = code[k][5];
+        V const *pxm = base(exm), *pxp = base(exp_), *pym = base(eym), *pyp = base(eyp);
+        T const *pot = ((iloc < 0) ? zero : Vcell + size_t(iloc)*64) + zq*16;
+        V cur[16], acc[16];
 #pragma unroll
-        for (int yy = 0; yy < 4; ++yy) {
-            double2 const v = srow(sc, pl, zq*4 + yy, 0), u = srow(sc, pl, zq*4 + yy, 1);
-            cur[yy*4] = v.x; cur[yy*4 + 1] = v.y; cur[yy*4 + 2] = u.x; cur[yy*4 + 3] = u.y;
-        }
-        double acc[16];
+        for (int i = 0; i < 16; ++i) cur[i] = mine[sc*SLOT + i*16];
         // potential and centre; the other plane of the own points from the partner lane
-        int32_t const iloc = code[k][5];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            double const V = (iloc < 0) ? 0.0 : __ldg(Vcell + size_t(iloc)*64 + zq*16 + i);
-            double const w = __shfl_xor_sync(0xffffffffu, cur[i], 16);
-            acc[i] = (V - a.E_re)*cur[i] + Eim*w + c0*cur[i];
+        for (int i = 0; i < 16; ++i)
+            acc[i] = vfma(vdup(__ldg(pot + i) + shift), cur[i], vmul(eim, __shfl_xor_sync(0xffffffffu, cur[i], 16)));
+        // z-stencil from the three staged cubes
+#pragma unroll
+        for (int d = 1; d <= 4; ++d) {
+            int const zm = zq - d, zp = zq + d;
+            V const *m = slots + ((zm < 0) ? sp : sc)*SLOT + (pl*64 + (zm & 3)*16)*16 + j;
+            V const *p = slots + ((zp > 3) ? sn : sc)*SLOT + (pl*64 + (zp & 3)*16)*16 + j;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[i] = vfma(cz[d], vadd(m[i*16], p[i*16]), acc[i]);
         }
+        __syncthreads();                                       // the previous cube is done with
+        if (k + 1 < n) fetch(sp, code[k + 1][6]);              // arrives during the rest of this step
         // y-stencil inside the cube
 #pragma unroll
         for (int yy = 0; yy < 4; ++yy)
 #pragma unroll
             for (int yo = 0; yo < 4; ++yo) {
                 if (yo == yy) continue;
-                int const d = (yo > yy) ? yo - yy : yy - yo;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) acc[yy*4 + i] += cy[d]*cur[yo*4 + i];
+                for (int i = 0; i < 4; ++i) acc[yy*4 + i] = vfma(cy[(yo > yy) ? yo - yy : yy - yo], cur[yo*4 + i], acc[yy*4 + i]);
             }
         // x-stencil: the rows of the x-neighbours at (zq, yy)
-        int32_t const exm = code[k][1], exp_ = code[k][2], eym = code[k][3], eyp = code[k][4];
 #pragma unroll
         for (int yy = 0; yy < 4; ++yy) {
-            double xm[4], xp[4];
+            V l[12];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                xm[i] = (-1 == exm) ? 0.0 : __ldg(x + size_t(nbr_block(exm))*kBlockReals + pl*4096 + (zq*16 + yy*4 + i)*64 + col);
-                xp[i] = (-1 == exp_) ? 0.0 : __ldg(x + size_t(nbr_block(exp_))*kBlockReals + pl*4096 + (zq*16 + yy*4 + i)*64 + col);
-            }
+            for (int i = 0; i < 4; ++i) { l[i] = __ldg(pxm + (yy*4 + i)*S); l[4 + i] = cur[yy*4 + i]; l[8 + i] = __ldg(pxp + (yy*4 + i)*S); }
             if (exm < -1) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) xm[i] = phase64(xm[i], pl, a.ph[0][0][0], a.ph[0][0][1]);
+                for (int i = 0; i < 4; ++i) l[i] = phase(l[i], a.ph[0][0][0], a.ph[0][0][1]);
             }
             if (exp_ < -1) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) xp[i] = phase64(xp[i], pl, a.ph[0][1][0], a.ph[0][1][1]);
+                for (int i = 8; i < 12; ++i) l[i] = phase(l[i], a.ph[0][1][0], a.ph[0][1][1]);
             }
-            double l[12];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { l[i] = xm[i]; l[4 + i] = cur[yy*4 + i]; l[8 + i] = xp[i]; }
+            for (int d = 1; d <= 4; ++d)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int d = 1; d <= 4; ++d) acc[yy*4 + i] += cx[d]*(l[4 + i - d] + l[4 + i + d]);
+                for (int i = 0; i < 4; ++i) acc[yy*4 + i] = vfma(cx[d], vadd(l[4 + i - d], l[4 + i + d]), acc[yy*4 + i]);
         }
         // y-neighbour cubes: row yo of y- sits at y = yo - 4, row yo of y+ at y = yo + 4
 #pragma unroll
         for (int yo = 0; yo < 4; ++yo) {
-            double ym[4], yp[4];
+            V ym[4], yp[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                ym[i] = (-1 == eym) ? 0.0 : __ldg(x + size_t(nbr_block(eym))*kBlockReals + pl*4096 + (zq*16 + yo*4 + i)*64 + col);
-                yp[i] = (-1 == eyp) ? 0.0 : __ldg(x + size_t(nbr_block(eyp))*kBlockReals + pl*4096 + (zq*16 + yo*4 + i)*64 + col);
-            }
+            for (int i = 0; i < 4; ++i) { ym[i] = __ldg(pym + (yo*4 + i)*S); yp[i] = __ldg(pyp + (yo*4 + i)*S); }
             if (eym < -1) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) ym[i] = phase64(ym[i], pl, a.ph[1][0][0], a.ph[1][0][1]);
+                for (int i = 0; i < 4; ++i) ym[i] = phase(ym[i], a.ph[1][0][0], a.ph[1][0][1]);
             }
             if (eyp < -1) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) yp[i] = phase64(yp[i], pl, a.ph[1][1][0], a.ph[1][1][1]);
+                for (int i = 0; i < 4; ++i) yp[i] = phase(yp[i], a.ph[1][1][0], a.ph[1][1][1]);
             }
 #pragma unroll
             for (int yy = 0; yy < 4; ++yy) {
-                if (yy <= yo) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[yy*4 + i] += cy[yy - yo + 4]*ym[i];
-                }
-                if (yy >= yo) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[yy*4 + i] += cy[yo + 4 - yy]*yp[i];
+                for (int i = 0; i < 4; ++i) {
+                    if (yy <= yo) acc[yy*4 + i] = vfma(cy[(yy - yo + 4) & 7], ym[i], acc[yy*4 + i]);
+                    if (yy >= yo) acc[yy*4 + i] = vfma(cy[(yo + 4 - yy) & 7], yp[i], acc[yy*4 + i]);
                 }
             }
         }
-        // z-stencil from the three staged cubes (previous, current, next)
+        V *yb = reinterpret_cast<V*>(y + size_t(code[k][0])*kBlockReals + lo) + zq*16*S;
 #pragma unroll
-        for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-            for (int d = 1; d <= 4; ++d) {
-                int const zm = zq - d, zp = zq + d;
-                int const s_m = (zm < 0) ? sp : sc, s_p = (zp > 3) ? sn : sc;
-                int const r_m = (zm & 3)*4 + yy, r_p = (zp & 3)*4 + yy;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    double2 const m = srow(s_m, pl, r_m, h), p = srow(s_p, pl, r_p, h);
-                    acc[yy*4 + 2*h] += cz[d]*(m.x + p.x);
-                    acc[yy*4 + 2*h + 1] += cz[d]*(m.y + p.y);
-                }
-            }
-        double *yb = y + size_t(b)*kBlockReals + pl*4096 + (zq*16)*64 + col;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) yb[i*64] = acc[i];
-        int const t = sp; sp = sc; sc = sn; sn = t;  // rotate the z-slots
+        for (int i = 0; i < 16; ++i) yb[i*S] = acc[i];
+        if (k + 1 < n) {
+            land();                                            // the cube after the next one
+            if (code[k + 1][6] < -1) { turn(sp, a.ph[2][1]); __syncthreads(); }
+        }
+        int const t = sp; sp = sc; sc = sn; sn = t;            // rotate the z-slots
     }
-}
-
-// Pencils with staged lateral cubes (FP32): the thread mapping and arithmetic of
-// local_pencil_kernel, but the four x- and y-neighbour cubes of step k + 1 are copied into shared
-// memory with 16-byte cp.async while step k is computed, so the stencil reads only shared memory
-// and registers and the neighbour rows' L2 latency is hidden behind a whole step.  The lateral
-// stage holds [2 steps][x-, x+, y-, y+][re, im][64 rows][32 columns]; one CTA per SM.
-constexpr int kStageLat = 4*2*64*kPencilS;                       // floats of one step's laterals
-constexpr int kStageSmem = kPencilSmem + 2*kStageLat*4;          // bytes: z-slots + two lateral steps
-
-__device__ __forceinline__ uint32_t smem_addr_u32(void const *p) { return uint32_t(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void cp_async16_cg(void *dst, void const *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_addr_u32(dst)), "l"(src) : "memory");
-}
-
-__global__ void __launch_bounds__(4*kPencilS, 1)
-local_stage_kernel(float *__restrict__ y, float const *__restrict__ x,
-                   uint32_t const *__restrict__ zstart, int32_t const *__restrict__ zlist,
-                   int32_t const *__restrict__ nbr, int32_t const *__restrict__ veff,
-                   float const *__restrict__ Vcell, LocalArgs<float> a)
-{
-    constexpr int S = kPencilS, NSL = 64/S;
-    extern __shared__ __align__(16) float4 slot4[];   // [3][2][16][S] float4, then the lateral stages
-    float *lat = reinterpret_cast<float*>(slot4 + 3*2*16*S);
-    __shared__ int32_t code[kMaxLine][8];              // per step: block, x-, x+, y-, y+, veff, z-next
-    __shared__ int32_t zleft, nline;
-    int const line = blockIdx.x/NSL, slice = blockIdx.x % NSL;
-    int const tid = threadIdx.x, j = tid % S, zq = tid/S, col = slice*S + j;
-    int32_t const *L = zlist + zstart[line];
-    if (0 == tid) {
-        int n = 0;
-        while (L[4 + n] > 0) ++n;                   // lists end with 4 non-positive entries
-        nline = n; zleft = list_code(L[3]);
-    }
-    __syncthreads();
-    int const n = nline;
-    if (0 == n || !line_args(a, L[4] - 1)) return;  // uniform: nothing on this line, or retired
-    for (int k = tid; k < n; k += 4*S) {
-        int32_t const b = L[4 + k] - 1;
-        int32_t const *nb = nbr + 6*size_t(b);
-        code[k][0] = b; code[k][1] = nb[0]; code[k][2] = nb[1]; code[k][3] = nb[2]; code[k][4] = nb[3];
-        code[k][5] = veff[b]; code[k][6] = list_code(L[5 + k]);
-    }
-    __syncthreads();                                // code[] complete
-    // the four lateral cubes of step k into stage st: 1024 16-byte pieces each, 8 per thread
-    auto issue = [&](int k, int st) {
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            int32_t const e = code[k][1 + l];
-            if (-1 == e) continue;                  // no cube: read as zeros, nothing to copy
-            float const *src = x + size_t(nbr_block(e))*kBlockReals + slice*S;
-            float *dst = lat + (st*4 + l)*2*64*S;
-#pragma unroll
-            for (int q = 0; q < 2*64*(S/4)/(4*S); ++q) {
-                int const c = q*4*S + tid;          // piece: (plane*64 + row)*(S/4) + quad
-                int const pr = c/(S/4), qd = c % (S/4);
-                cp_async16_cg(dst + pr*S + qd*4, src + pr*64 + qd*4);
-            }
-        }
-    };
-    auto srow = [&](int slot, int pl, int row) -> float4 & { return slot4[((slot*2 + pl)*16 + row)*S + j]; };
-    auto put = [&](int slot, Quad const &q) {
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-            for (int pl = 0; pl < 2; ++pl)
-                srow(slot, pl, zq*4 + yy) = make_float4(q.v[pl][yy*4], q.v[pl][yy*4 + 1], q.v[pl][yy*4 + 2], q.v[pl][yy*4 + 3]);
-    };
-    // row (zq, r4) of lateral l of stage st: 4 x-points, re and im, with the Bloch phase of its code
-    auto lrow = [&](int st, int l, int r4, int32_t e, float pr, float pi, Rows<float> &o) {
-        if (-1 == e) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) { o.re[i] = 0.f; o.im[i] = 0.f; }
-            return;
-        }
-        float const *b = lat + (st*4 + l)*2*64*S + (zq*16 + r4*4)*S + j;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) { o.re[i] = b[i*S]; o.im[i] = b[64*S + i*S]; }
-        row_phase(e, pr, pi, o);
-    };
-    float const (&cx)[5] = a.st.c[0];
-    float const (&cy)[5] = a.st.c[1];
-    float const (&cz)[5] = a.st.c[2];
-    float const c0 = cx[0] + cy[0] + cz[0];
-    issue(0, 0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    {
-        Quad h;
-        quad_raw(x, zleft, zq, col, h);
-        quad_phase(zleft, a.ph[2][0][0], a.ph[2][0][1], h);
-        put(0, h);
-        quad_raw(x, code[0][0], zq, col, h);
-        put(1, h);
-    }
-    Quad nx;                                        // rows of the z-successor, one step ahead
-    quad_raw(x, code[0][6], zq, col, nx);
-    int sp = 0, sc = 1, sn = 2;
-    for (int k = 0; k < n; ++k) {
-        int32_t const b = code[k][0];
-        int const st = k & 1;
-        quad_phase(code[k][6], a.ph[2][1][0], a.ph[2][1][1], nx);   // only the line end has a phase
-        __syncthreads();                            // step k-1 finished reading slot sn and stage st^1
-        if (k + 1 < n) issue(k + 1, st ^ 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        put(sn, nx);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");   // this thread's copies of step k landed
-        __syncthreads();                            // ... and everybody else's; slot sn written
-        if (k + 1 < n) quad_raw(x, code[k + 1][6], zq, col, nx);   // arrives during this step
-        Quad cur;
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-            for (int pl = 0; pl < 2; ++pl) {
-                float4 const v = srow(sc, pl, zq*4 + yy);
-                cur.v[pl][yy*4] = v.x; cur.v[pl][yy*4 + 1] = v.y; cur.v[pl][yy*4 + 2] = v.z; cur.v[pl][yy*4 + 3] = v.w;
-            }
-        float acc[2][16];
-        int32_t const iloc = code[k][5];
-        float V[16];
-        if (iloc < 0) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) V[i] = 0.f;
-        } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float4 const v = __ldg(reinterpret_cast<float4 const*>(Vcell + size_t(iloc)*64 + zq*16 + q*4));
-                V[q*4] = v.x; V[q*4 + 1] = v.y; V[q*4 + 2] = v.z; V[q*4 + 3] = v.w;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            float const Vt = V[i] - a.E_re;
-            acc[0][i] = Vt*cur.v[0][i] + a.E_im*cur.v[1][i] + c0*cur.v[0][i];
-            acc[1][i] = Vt*cur.v[1][i] - a.E_im*cur.v[0][i] + c0*cur.v[1][i];
-        }
-#pragma unroll
-        for (int pl = 0; pl < 2; ++pl)
-#pragma unroll
-            for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-                for (int yo = 0; yo < 4; ++yo) {
-                    if (yo == yy) continue;
-                    int const d = (yo > yy) ? yo - yy : yy - yo;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[pl][yy*4 + i] += cy[d]*cur.v[pl][yo*4 + i];
-                }
-        int32_t const exm = code[k][1], exp_ = code[k][2], eym = code[k][3], eyp = code[k][4];
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy) {
-            Rows<float> xm, xp;
-            lrow(st, 0, yy, exm, a.ph[0][0][0], a.ph[0][0][1], xm);
-            lrow(st, 1, yy, exp_, a.ph[0][1][0], a.ph[0][1][1], xp);
-            float lr[12], li[12];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                lr[i] = xm.re[i]; li[i] = xm.im[i];
-                lr[4 + i] = cur.v[0][yy*4 + i]; li[4 + i] = cur.v[1][yy*4 + i];
-                lr[8 + i] = xp.re[i]; li[8 + i] = xp.im[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int d = 1; d <= 4; ++d) {
-                    acc[0][yy*4 + i] += cx[d]*(lr[4 + i - d] + lr[4 + i + d]);
-                    acc[1][yy*4 + i] += cx[d]*(li[4 + i - d] + li[4 + i + d]);
-                }
-        }
-#pragma unroll
-        for (int yo = 0; yo < 4; ++yo) {
-            Rows<float> ym, yp;
-            lrow(st, 2, yo, eym, a.ph[1][0][0], a.ph[1][0][1], ym);
-            lrow(st, 3, yo, eyp, a.ph[1][1][0], a.ph[1][1][1], yp);
-#pragma unroll
-            for (int yy = 0; yy < 4; ++yy) {
-                if (yy <= yo) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        acc[0][yy*4 + i] += cy[yy - yo + 4]*ym.re[i];
-                        acc[1][yy*4 + i] += cy[yy - yo + 4]*ym.im[i];
-                    }
-                }
-                if (yy >= yo) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        acc[0][yy*4 + i] += cy[yo + 4 - yy]*yp.re[i];
-                        acc[1][yy*4 + i] += cy[yo + 4 - yy]*yp.im[i];
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int yy = 0; yy < 4; ++yy)
-#pragma unroll
-            for (int d = 1; d <= 4; ++d) {
-                int const zm = zq - d, zp = zq + d;
-                int const s_m = (zm < 0) ? sp : sc, s_p = (zp > 3) ? sn : sc;
-                int const r_m = (zm & 3)*4 + yy, r_p = (zp & 3)*4 + yy;
-#pragma unroll
-                for (int pl = 0; pl < 2; ++pl) {
-                    float4 const m = srow(s_m, pl, r_m), p = srow(s_p, pl, r_p);
-                    acc[pl][yy*4 + 0] += cz[d]*(m.x + p.x);
-                    acc[pl][yy*4 + 1] += cz[d]*(m.y + p.y);
-                    acc[pl][yy*4 + 2] += cz[d]*(m.z + p.z);
-                    acc[pl][yy*4 + 3] += cz[d]*(m.w + p.w);
-                }
-            }
-        float *yb = y + size_t(b)*kBlockReals + (zq*16)*64 + col;
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { yb[i*64] = acc[0][i]; yb[4096 + i*64] = acc[1][i]; }
-        int const t = sp; sp = sc; sc = sn; sn = t;  // rotate the z-slots
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // ---------------------------------------------------------------- generic local path
@@ -1478,9 +879,8 @@ void launch_project_L(DevicePlan &dp, T const *x, cudaStream_t st) {
 
 bool prepare_local_kernels() {
     // the pencil kernel's three z-slots are 48 KB of dynamic shared memory beside its static part
-    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
-    A43G_CUDA_TRY(cudaFuncSetAttribute(local_stage_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageSmem));
-    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencil64Smem));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
     return true;
 }
 
@@ -1507,38 +907,13 @@ bool launch_local(DevicePlan &dp, T *y, T const *x, cudaStream_t st) {
     if (dp.fused_local) {
         constexpr int S = (sizeof(T) == 8) ? 8 : 16;
         unsigned const nblk = dp.nlists[2]*(64/S);
-        if constexpr (sizeof(T) == 4) {
-            if (dp.nlists[2] && dp.max_zline <= kMaxLine && 3 == dp.local_variant &&
-                0 == (reinterpret_cast<uintptr_t>(x) & 15u)) {
-                local_stage_kernel<<<dp.nlists[2]*(64/kPencilS), 4*kPencilS, kStageSmem, st>>>(y, x,
-                    dptr<uint32_t>(dp.lists_start[2]), dptr<int32_t>(dp.lists[2]), dptr<int32_t>(dp.nbr),
-                    dptr<int32_t>(dp.veff_index), vcell<T>(dp), a);
-                count_launch();
-                A43G_CUDA_TRY(cudaGetLastError());
-                return true;
-            }
-            if (dp.nlists[2] && dp.max_zline <= kMaxLine && (2 == dp.local_variant || 3 == dp.local_variant)) {
-                local_pencil_kernel<<<dp.nlists[2]*(64/kPencilS), 4*kPencilS, kPencilSmem, st>>>(y, x,
-                    dptr<uint32_t>(dp.lists_start[2]), dptr<int32_t>(dp.lists[2]), dptr<int32_t>(dp.nbr),
-                    dptr<int32_t>(dp.veff_index), vcell<T>(dp), a);
-                count_launch();
-                A43G_CUDA_TRY(cudaGetLastError());
-                return true;
-            }
-        }
-        if constexpr (sizeof(T) == 8) {
-            if (dp.nlists[2] && dp.max_zline <= kMaxLine && dp.local64_pencils) {
-                local_pencil64_kernel<<<dp.nlists[2]*(64/kPencil64S), 8*kPencil64S, kPencil64Smem, st>>>(y, x,
-                    dptr<uint32_t>(dp.lists_start[2]), dptr<int32_t>(dp.lists[2]), dptr<int32_t>(dp.nbr),
-                    dptr<int32_t>(dp.veff_index), vcell<T>(dp), a);
-                count_launch();
-                A43G_CUDA_TRY(cudaGetLastError());
-                return true;
-            }
-        }
-        if (nblk && sizeof(T) == 4 && dp.max_zline <= kMaxLine && 0 == dp.local_variant) {
-            local_fused_pf_kernel<T, S><<<nblk, S*16, 0, st>>>(y, x, dptr<uint32_t>(dp.lists_start[2]),
-                dptr<int32_t>(dp.lists[2]), dptr<int32_t>(dp.nbr), dptr<int32_t>(dp.veff_index), vcell<T>(dp), a);
+        // pencils copy 16 bytes at a time and hold the codes of a line; the rows kernel takes the
+        // other calls
+        bool const pencils = !dp.local_rows && dp.max_zline <= kMaxLine && vectors_aligned16(x, y);
+        if (nblk && pencils) {
+            local_pencil_kernel<T><<<dp.nlists[2]*(unsigned(sizeof(T))/2), kPencilThreads, kPencilSmem, st>>>(y, x,
+                dptr<uint32_t>(dp.lists_start[2]), dptr<int32_t>(dp.lists[2]), dptr<int32_t>(dp.nbr),
+                dptr<int32_t>(dp.veff_index), vcell<T>(dp), dptr<T>(dp.zero_block), a);
             count_launch();
         } else if (nblk) {
             local_fused_kernel<T, S><<<nblk, S*16, 0, st>>>(y, x, dptr<uint32_t>(dp.lists_start[2]),
@@ -1584,7 +959,7 @@ bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, c
     // both FP32 projector paths stage x with 16-byte loads; other x take the generic kernels
     bool const aligned16 = 0 == (reinterpret_cast<uintptr_t>(x) & 15u);
     bool const tc = (sizeof(T) == 4) && dp.use_tc && aligned16 && tc_projector_supported(dp);
-    bool const lines = !tc && line_projector_supported(x, y);
+    bool const lines = !tc && vectors_aligned16(x, y);
     if (tc) {
         if (!launch_project_tc(dp, (float const*)x, st)) return false;
     } else if (lines) {

@@ -5,10 +5,7 @@
 //   * prj_chunk   : blocks of one (image, source) list per projection CTA (the cubes-per-CTA
 //                   schedule of the projection: longer chunks amortize the pipeline start and
 //                   the coefficient atomics, shorter ones balance the load)   {12, 24, 40}
-//   * local_variant: FP32 local kernel on rows with one-step-ahead loads, on plain rows, on
-//                   y-pencils, or on y-pencils with staged neighbour cubes     {0, 1, 2, 3}
 //   * use_tc      : FP32 projector on the tensor cores (3xTF32) or on the CUDA cores
-//   * local64_pencils: FP64 local kernel on pencils (planes on two threads) or on rows
 // Each parameter is tuned in turn (coordinate descent), every candidate timed with CUDA events
 // on the caller's stream: two untimed applications, then the mean of three.  Scratch vectors
 // for x and y are allocated for the duration of the call.
@@ -88,32 +85,8 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
             }
         }
     }
-    char const *const local_name[4] = {"rows with loads ahead", "plain rows", "pencils", "staged pencils"};
-    if (sizeof(T) == 4 && dp.fused_local) {
-        float t[4] = {0, 0, 0, 0};
-        int best = 0;
-        for (int v = 0; v < 4; ++v) {
-            dp.local_variant = v;
-            if (!time_part<T>(dp, 0, y, x, ci, st, t[v])) return false;
-            std::snprintf(line, sizeof(line), "local kernel, %s: %.3f ms\n", local_name[v], t[v]);
-            report += line;
-            if (t[v] < t[best]) best = v;
-        }
-        dp.local_variant = best;
-    }
-    if (sizeof(T) == 8 && dp.fused_local) {
-        float t[2] = {0, 0};
-        for (int v = 0; v < 2; ++v) {
-            dp.local64_pencils = (1 == v);
-            if (!time_part<T>(dp, 0, y, x, ci, st, t[v])) return false;
-            std::snprintf(line, sizeof(line), "FP64 local kernel, %s: %.3f ms\n", v ? "pencils" : "rows", t[v]);
-            report += line;
-        }
-        dp.local64_pencils = t[1] <= t[0];
-    }
-    std::snprintf(line, sizeof(line), "chosen: projector chunk %u, local %s, %s projector\n",
-                  dp.prj_chunk, local_name[dp.local_variant],
-                  dp.use_tc ? "tensor-core" : "CUDA-core");
+    std::snprintf(line, sizeof(line), "chosen: projector chunk %u, %s projector\n",
+                  dp.prj_chunk, dp.use_tc ? "tensor-core" : "CUDA-core");
     report += line;
     A43G_CUDA_TRY(cudaStreamSynchronize(st));
     return true;

@@ -66,8 +66,7 @@ struct DevicePlan {
     uint32_t max_zline = 0;      // cubes in the longest z-line
     // schedule parameters, set by the autotuner (autotune.cu) or left at these defaults
     uint32_t prj_chunk = 0;          // blocks per projection work item (0: by the plan's size)
-    int local_variant = 2;           // FP32: 0 rows with one-step-ahead loads, 1 plain rows, 2 pencils, 3 staged pencils
-    bool local64_pencils = true;     // FP64: pencils with the planes on two threads, else the row kernel
+    bool local_rows = false;         // the local part by the rows kernel
     bool atom_chain3 = false;        // atom matrices by the collect/multiply/broadcast kernels instead of one
     uint32_t nlists[3] = {0, 0, 0};
 
@@ -75,6 +74,7 @@ struct DevicePlan {
     DeviceBuffer Vcell64, Vcell32;  // [ncells][64]
     DeviceBuffer nbr;            // int32 [nnzb][6]  x-, x+, y-, y+, z-, z+
     DeviceBuffer lists_start[3], lists[3];
+    DeviceBuffer zero_block;     // a block of zeros: neighbours that do not exist
     DeviceBuffer colindx;        // uint16 [nnzb]
     DeviceBuffer rowindx;        // uint32 [nnzb]
     DeviceBuffer rowCubePos;     // float [nRows][4]
@@ -173,9 +173,9 @@ bool tc_projector_supported(DevicePlan const &dp);
 bool launch_project_tc(DevicePlan &dp, float const *x, cudaStream_t st);
 bool launch_add_tc(DevicePlan &dp, float *y, uint16_t const *colIndex, cudaStream_t st);
 
-// projection and addition along lines of cubes on the CUDA cores (projector_line.cuh); x and y on
-// 16-byte boundaries (the kernels move 8 bytes per lane)
-inline bool line_projector_supported(void const *x, void const *y) {
+// vectors that the kernels on 8-byte lanes with 16-byte copies take (local pencils; projection and
+// addition along lines of cubes, projector_line.cuh)
+inline bool vectors_aligned16(void const *x, void const *y) {
     return 0 == ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u);
 }
 // the projection along lines with the given tables (every coefficient of an active source is written)

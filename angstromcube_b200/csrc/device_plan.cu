@@ -107,6 +107,8 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
 
     if (!put(dp.veff_index, hp.veff_index)) return false;
     if (!put(dp.nbr, neighbour_table(hp))) return false;
+    if (!dp.zero_block.alloc(8192*sizeof(double))) return false;
+    A43G_CUDA_TRY(cudaMemset(dp.zero_block.ptr, 0, 8192*sizeof(double)));
     for (int d = 0; d < 3; ++d) {
         if (!put(dp.lists_start[d], hp.kinetic[d].start)) return false;
         if (!put(dp.lists[d], hp.kinetic[d].entry)) return false;
@@ -184,14 +186,10 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
         // FP32 projector: SIMT (default) or the tensor cores ("tc"); the FP64 path is always SIMT
         char const *e = std::getenv("A43G_PROJECTOR");
         dp.use_tc = (e && 0 == std::strcmp(e, "tc"));
-        // FP32 local kernel: y-"pencils" (default), pencils with "staged" neighbour cubes, "rows"
-        // with loads ahead or "plain" rows
-        char const *l = std::getenv("A43G_LOCAL");
-        dp.local_variant = (l && 0 == std::strcmp(l, "plain")) ? 1 : ((l && 0 == std::strcmp(l, "rows")) ? 0 :
-                           ((l && 0 == std::strcmp(l, "staged")) ? 3 : 2));
-        // FP64 local kernel: "pencils" (default) or "rows"
-        char const *l64 = std::getenv("A43G_LOCAL64");
-        dp.local64_pencils = !(l64 && 0 == std::strcmp(l64, "rows"));
+        // local kernel: pencils (default) or "rows" ("plain" in FP32), the kernel of unaligned vectors
+        char const *l = std::getenv("A43G_LOCAL"), *l64 = std::getenv("A43G_LOCAL64");
+        dp.local_rows = (l && (0 == std::strcmp(l, "rows") || 0 == std::strcmp(l, "plain"))) ||
+                        (l64 && 0 == std::strcmp(l64, "rows"));
         // atom-matrix chain: one kernel (default) or "three" (collect, multiply, broadcast)
         char const *ac = std::getenv("A43G_ATOM_CHAIN");
         dp.atom_chain3 = (ac && 0 == std::strcmp(ac, "three"));

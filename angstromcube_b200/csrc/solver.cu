@@ -1523,7 +1523,7 @@ int solve_batched(GreenPlan &hp, DevicePlan &dp, BatchCache &bc, a43g_solve_opti
         bc.ws.reset(new SolverWorkspace());
         bc.dev->prj_chunk = dp.prj_chunk;
         if (!upload_plan(bc.host, *bc.dev)) return A43G_ERR_CUDA;
-        bc.dev->local_variant = dp.local_variant; bc.dev->use_tc = dp.use_tc;
+        bc.dev->use_tc = dp.use_tc;
         bc.npairs = wave;
     }
     // the caller's potential and atom matrices as they are now
