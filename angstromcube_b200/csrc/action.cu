@@ -616,7 +616,7 @@ sho_project_kernel(T *__restrict__ apc, T const *__restrict__ x, uint32_t nrhs,
 }
 
 // aac[(a0 + c)*nrhs + s] = sum over the images i of atom A of phase_i * apc[(i0 + c)*nrhs + s]
-// (collect) in double (include/green_dyadic.hxx:600-702).  Grid (nAtoms, nrhs), 64 threads.
+// (collect) in double (include/green_dyadic.hxx:600-702).  Grid (nAtoms, nrhs, rows), 64 threads.
 // per-source selection of the pair values of a batch plan (image phases and atom matrices
 // stored [pair][...]) and the retirement flags (nullptr: every source active)
 struct DyadicPairs {
@@ -638,7 +638,7 @@ sho_collect_kernel(double *__restrict__ aac, T const *__restrict__ apc, uint32_t
     img_phase += (s/bp.nsrc_pair)*bp.img_stride;
     int const nc = nsho_c(atom_lmax[A]);
     size_t const a0 = atom_starts[A];
-    for (int c = 0; c < nc; ++c) {
+    for (int c = blockIdx.z; c < nc; c += gridDim.z) {
         double re = 0, im = 0;
         for (uint32_t k = sum_start[A]; k < sum_start[A + 1]; ++k) {
             uint32_t const i = sum_col[k];
@@ -653,8 +653,10 @@ sho_collect_kernel(double *__restrict__ aac, T const *__restrict__ apc, uint32_t
     }
 }
 
+constexpr int kMulRows = 8;
+
 // out[(a0 + i)*nrhs + s] = sum_k M_A[i][k] in[(a0 + k)*nrhs + s], complex, accumulated in
-// double (include/green_dyadic.hxx:740-826).  Grid (nAtoms, nrhs), 64 threads.
+// double (include/green_dyadic.hxx:740-826).  Grid (nAtoms, nrhs, groups of 8 rows), 64 threads.
 template <typename Tin, typename Tout>
 __global__ void __launch_bounds__(64)
 sho_mul_kernel(Tout *__restrict__ out, Tin const *__restrict__ in, uint32_t nrhs,
@@ -667,8 +669,8 @@ sho_mul_kernel(Tout *__restrict__ out, Tin const *__restrict__ in, uint32_t nrhs
     int const nc = nsho_c(atom_lmax[A]);
     size_t const a0 = atom_starts[A];
     double const *Mr = mats + mat_off[A], *Mi = Mr + nc*nc;
-    constexpr int R = 8;                       // output rows per pass: each input value is loaded once per R rows
-    for (int i0 = 0; i0 < nc; i0 += R) {
+    constexpr int R = kMulRows;                // output rows per pass: each input value is loaded once per R rows
+    for (int i0 = blockIdx.z*R; i0 < nc; i0 += gridDim.z*R) {
         double re[R], im[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) { re[r] = 0; im[r] = 0; }
@@ -693,7 +695,7 @@ sho_mul_kernel(Tout *__restrict__ out, Tin const *__restrict__ in, uint32_t nrhs
 }
 
 // cad[(i0 + c)*nrhs + s] = conj(phase_i) * cadd[(a0 + c)*nrhs + s] for every image i of atom A
-// (broadcast, include/green_dyadic.hxx:683-694).  Grid (nAtoms, nrhs), 64 threads.
+// (broadcast, include/green_dyadic.hxx:683-694).  Grid (nAtoms, nrhs, rows), 64 threads.
 template <typename T>
 __global__ void __launch_bounds__(64)
 sho_broadcast_kernel(T *__restrict__ cad, double const *__restrict__ cadd, uint32_t nrhs,
@@ -710,7 +712,7 @@ sho_broadcast_kernel(T *__restrict__ cad, double const *__restrict__ cadd, uint3
     for (uint32_t k = sum_start[A]; k < sum_start[A + 1]; ++k) {
         uint32_t const i = sum_col[k];
         double const pr = img_phase[4*i], pi = -img_phase[4*i + 1];
-        for (int c = 0; c < nc; ++c) {
+        for (int c = blockIdx.z; c < nc; c += gridDim.z) {
             double const *src = cadd + ((a0 + c)*nrhs + s)*128;
             double const xr = src[j], xi = src[64 + j];
             T *dst = cad + ((size_t(img_starts[i]) + c)*nrhs + s)*128;
@@ -871,6 +873,12 @@ sho_add_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs, uint
     for (int p = 0; p < 64; ++p) if ((mask_all >> p) & 1) yb[p*64] += acc[p];
 }
 
+// grids of the three-kernel chain: the rows of an atom over the z-index, 4 rows per CTA (a plan of 64
+// atoms and one source would keep 64 CTAs busy with 56 rows each: 239 us against 31 for the collect
+// kernel)
+dim3 row_grid(DevicePlan const &dp) { return dim3(dp.nAtoms, dp.nCols, unsigned((nsho_c(std::max(dp.lmax_max, 0)) + 3)/4)); }
+dim3 mul_grid(DevicePlan const &dp) { return dim3(dp.nAtoms, dp.nCols, unsigned((nsho_c(std::max(dp.lmax_max, 0)) + kMulRows - 1)/kMulRows)); }
+
 DyadicPairs dyadic_pairs(DevicePlan const &dp) {
     DyadicPairs bp;
     bp.nsrc_pair = dp.nsrc_pair ? dp.nsrc_pair : std::max(1u, dp.nCols);
@@ -991,7 +999,8 @@ bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, c
         if (!launch_project_tc(dp, (float const*)x, st)) return false;
     } else if (lines) {
         if (!ensure_prj_part(dp, sizeof(T))) return false;
-        if (!launch_project_line(dp, dptr<T>(dp.apc), x, sizeof(T) == 8 ? dp.line_tab64.ptr : dp.line_tab32.ptr, st)) return false;
+        if (!launch_project_line(dp, dptr<T>(dp.apc), x, sizeof(T) == 8 ? dp.line_tab64.ptr : dp.line_tab32.ptr,
+                                 LineScratch{dp.prj_part.ptr, dptr<uint32_t>(dp.prj_line.tickets)}, st)) return false;
     } else {
         // coefficients of images without any block stay zero
         A43G_CUDA_TRY(cudaMemsetAsync(dp.apc.ptr, 0, size_t(dp.ncoeffI)*dp.nCols*128*sizeof(T), st));
@@ -1000,7 +1009,7 @@ bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, c
         launch_project_L<T, 4>(dp, x, st); launch_project_L<T, 5>(dp, x, st);
         launch_project_L<T, 6>(dp, x, st); launch_project_L<T, 7>(dp, x, st);
     }
-    dim3 const ga(dp.nAtoms, dp.nCols);
+    dim3 const ga = row_grid(dp), gm = mul_grid(dp);
     if (dp.lmax_max <= 5 && !dp.atom_chain3) {
         sho_atom_kernel<T><<<dim3(dp.nAtoms, dp.nCols, 2), 128, 0, st>>>(dptr<T>(dp.cad), dptr<T>(dp.apc), dp.nCols,
             dptr<int8_t>(dp.atom_lmax), dptr<uint32_t>(dp.sum_start), dptr<uint32_t>(dp.sum_col),
@@ -1012,7 +1021,7 @@ bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, c
             dptr<uint32_t>(dp.atom_starts), dptr<int8_t>(dp.atom_lmax), dptr<uint32_t>(dp.sum_start),
             dptr<uint32_t>(dp.sum_col), dptr<uint32_t>(dp.img_starts), dptr<double>(dp.img_phase), dyadic_pairs(dp));
         count_launch();
-        sho_mul_kernel<double, double><<<ga, 64, 0, st>>>(dptr<double>(dp.cadd), dptr<double>(dp.aac), dp.nCols,
+        sho_mul_kernel<double, double><<<gm, 64, 0, st>>>(dptr<double>(dp.cadd), dptr<double>(dp.aac), dp.nCols,
             dptr<uint32_t>(dp.atom_starts), dptr<int8_t>(dp.atom_lmax), dptr<double>(dp.atom_mat), dptr<uint32_t>(dp.atom_mat_off), dyadic_pairs(dp));
         count_launch();
         sho_broadcast_kernel<T><<<ga, 64, 0, st>>>(dptr<T>(dp.cad), dptr<double>(dp.cadd), dp.nCols,
@@ -1020,7 +1029,7 @@ bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, c
             dptr<uint32_t>(dp.sum_col), dptr<uint32_t>(dp.img_starts), dptr<double>(dp.img_phase), dyadic_pairs(dp));
         count_launch();
     } else {
-        sho_mul_kernel<T, T><<<ga, 64, 0, st>>>(dptr<T>(dp.cad), dptr<T>(dp.apc), dp.nCols,
+        sho_mul_kernel<T, T><<<gm, 64, 0, st>>>(dptr<T>(dp.cad), dptr<T>(dp.apc), dp.nCols,
             dptr<uint32_t>(dp.atom_starts), dptr<int8_t>(dp.atom_lmax), dptr<double>(dp.atom_mat), dptr<uint32_t>(dp.atom_mat_off), dyadic_pairs(dp));
         count_launch();
     }
@@ -1072,12 +1081,8 @@ bool project_into(DevicePlan &dp, T *apc, T const *x, double const *table, cudaS
 }
 } // namespace
 
-bool launch_project_with(DevicePlan &dp, double *apc, double const *x, double const *table, cudaStream_t st) {
-    return project_into<double>(dp, apc, x, table, st);
-}
-
 bool launch_collect_with(DevicePlan &dp, double *aac, double const *apc, double const *img_phase, cudaStream_t st) {
-    dim3 const ga(dp.nAtoms, dp.nCols);
+    dim3 const ga = row_grid(dp);
     sho_collect_kernel<double><<<ga, 64, 0, st>>>(aac, apc, dp.nCols, dptr<uint32_t>(dp.atom_starts),
         dptr<int8_t>(dp.atom_lmax), dptr<uint32_t>(dp.sum_start), dptr<uint32_t>(dp.sum_col),
         dptr<uint32_t>(dp.img_starts), img_phase, dyadic_pairs(dp));
@@ -1087,8 +1092,8 @@ bool launch_collect_with(DevicePlan &dp, double *aac, double const *apc, double 
 }
 
 bool launch_mul_with(DevicePlan &dp, double *out, double const *in, cudaStream_t st) {
-    dim3 const ga(dp.nAtoms, dp.nCols);
-    sho_mul_kernel<double, double><<<ga, 64, 0, st>>>(out, in, dp.nCols, dptr<uint32_t>(dp.atom_starts),
+    dim3 const gm = mul_grid(dp);
+    sho_mul_kernel<double, double><<<gm, 64, 0, st>>>(out, in, dp.nCols, dptr<uint32_t>(dp.atom_starts),
         dptr<int8_t>(dp.atom_lmax), dptr<double>(dp.atom_mat), dptr<uint32_t>(dp.atom_mat_off), dyadic_pairs(dp));
     count_launch();
     A43G_CUDA_TRY(cudaGetLastError());
@@ -1103,13 +1108,13 @@ bool launch_action_scratch(DevicePlan &dp, T *y, T const *x, uint16_t const *col
     if (dp.nAI < 1 || dp.nCols < 1) return true;
     T *apc = static_cast<T*>(sc.apc), *cad = static_cast<T*>(sc.cad);
     if (!project_into<T>(dp, apc, x, dptr<double>(dp.slot_H), st)) return false;
-    dim3 const ga(dp.nAtoms, dp.nCols);
+    dim3 const ga = row_grid(dp), gm = mul_grid(dp);
     if (dp.nAI > dp.nAtoms) {
         sho_collect_kernel<T><<<ga, 64, 0, st>>>(sc.aac, apc, dp.nCols,
             dptr<uint32_t>(dp.atom_starts), dptr<int8_t>(dp.atom_lmax), dptr<uint32_t>(dp.sum_start),
             dptr<uint32_t>(dp.sum_col), dptr<uint32_t>(dp.img_starts), dptr<double>(dp.img_phase), dyadic_pairs(dp));
         count_launch();
-        sho_mul_kernel<double, double><<<ga, 64, 0, st>>>(sc.cadd, sc.aac, dp.nCols,
+        sho_mul_kernel<double, double><<<gm, 64, 0, st>>>(sc.cadd, sc.aac, dp.nCols,
             dptr<uint32_t>(dp.atom_starts), dptr<int8_t>(dp.atom_lmax), dptr<double>(dp.atom_mat), dptr<uint32_t>(dp.atom_mat_off), dyadic_pairs(dp));
         count_launch();
         sho_broadcast_kernel<T><<<ga, 64, 0, st>>>(cad, sc.cadd, dp.nCols,
@@ -1117,7 +1122,7 @@ bool launch_action_scratch(DevicePlan &dp, T *y, T const *x, uint16_t const *col
             dptr<uint32_t>(dp.sum_col), dptr<uint32_t>(dp.img_starts), dptr<double>(dp.img_phase), dyadic_pairs(dp));
         count_launch();
     } else {
-        sho_mul_kernel<T, T><<<ga, 64, 0, st>>>(cad, apc, dp.nCols,
+        sho_mul_kernel<T, T><<<gm, 64, 0, st>>>(cad, apc, dp.nCols,
             dptr<uint32_t>(dp.atom_starts), dptr<int8_t>(dp.atom_lmax), dptr<double>(dp.atom_mat), dptr<uint32_t>(dp.atom_mat_off), dyadic_pairs(dp));
         count_launch();
     }

@@ -105,7 +105,9 @@ int projection_coefficients(GreenPlan const &hp, DevicePlan &dp, DensityWorkspac
     }
     if (!ws.apc.alloc(std::max<size_t>(16, nI*8)) || !ws.aac.alloc(std::max<size_t>(16, nA*8))) return A43G_ERR_MEMORY;
     // <p|G: the image projections and their phase-weighted sums onto the atoms
-    if (!launch_project_with(dp, dptr<double>(ws.apc), G, dptr<double>(dp.slot_H), st)) return A43G_ERR_CUDA;
+    LineScratch sc;
+    if (!ensure_line_scratch(dp, ws.lines, 8, st, sc)) return A43G_ERR_MEMORY;
+    if (!launch_project_line(dp, dptr<double>(ws.apc), G, dp.line_tab64.ptr, sc, st)) return A43G_ERR_CUDA;
     if (!launch_collect_with(dp, dptr<double>(ws.aac), dptr<double>(ws.apc), dptr<double>(dp.img_phase), st))
         return A43G_ERR_CUDA;
     dim3 const grid(dp.nAI, uint32_t(nsho(dp.lmax_max)));

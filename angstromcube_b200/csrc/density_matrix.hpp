@@ -11,6 +11,7 @@ struct DensityWorkspace {
     size_t nout = 0;                     // doubles of the result
     int stride = 0;                      // doubles per (image, source) table
     DeviceBuffer srcH, srcMask, out_off, out, img_index;
+    OwnLineScratch lines;
     DeviceBuffer apc, aac;               // image projections of G and their sums onto the atoms
 };
 

@@ -51,6 +51,9 @@ struct AddSegment { uint32_t blk[kSegment]; uint64_t any[kSegment]; uint32_t fir
 // slot (kNoSlot: not near) and the mask; the cubes share the y- and z-tables of yz_slot
 struct AddRecord { uint32_t coeff, lmax, slot[kSegment], yz_slot, pad; uint64_t mask[kSegment]; };
 
+// scratch of a projection outside the action (its own stream)
+struct OwnLineScratch { DeviceBuffer part, tickets; size_t groups = 0; };
+
 struct DevicePlan {
     bool uploaded = false;       // plan geometry on the device
     bool values_dirty = true;    // potential / matrices / phases need re-upload
@@ -98,7 +101,7 @@ struct DevicePlan {
     // the projection along lines (projector_line.cuh): items of every (image, source) pair, one
     // record {block, slot and flags, mask} per list position, and the slots' tables as
     // [dir][point][order] with 8 bytes per value (FP32: the value twice), the orders padded to even
-    struct PrjLine { uint32_t count = 0; size_t part_rows = 0; DeviceBuffer items, tickets; } prj_line;
+    struct PrjLine { uint32_t count = 0; size_t part_rows = 0, groups = 0; DeviceBuffer items, tickets; } prj_line;
     DeviceBuffer prj_rec, line_tab64, line_tab32;
     uint32_t nslots = 0;
     uint32_t add_segments = 0;   // the addition along lines: AddSegment, AddRecord
@@ -162,9 +165,7 @@ bool launch_action_scratch(DevicePlan &dp, T *y, T const *x, uint16_t const *col
                            DyadicScratch const &sc);
 
 // FP64 pieces of the dyadic part on caller-given buffers (vector-Jacobian products):
-// apc = P x with the given projector tables (zeroed first); aac = sum over images of
-// img_phase * apc; out = M in (atom matrices of the plan)
-bool launch_project_with(DevicePlan &dp, double *apc, double const *x, double const *table, cudaStream_t st);
+// aac = sum over images of img_phase * apc; out = M in (atom matrices of the plan)
 bool launch_collect_with(DevicePlan &dp, double *aac, double const *apc, double const *img_phase, cudaStream_t st);
 bool launch_mul_with(DevicePlan &dp, double *out, double const *in, cudaStream_t st);
 
@@ -178,9 +179,17 @@ bool launch_add_tc(DevicePlan &dp, float *y, uint16_t const *colIndex, cudaStrea
 inline bool vectors_aligned16(void const *x, void const *y) {
     return 0 == ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u);
 }
-// the projection along lines with the given tables (every coefficient of an active source is written)
-bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const *tab, cudaStream_t st);
-bool launch_project_line(DevicePlan &dp, double *apc, double const *x, void const *tab, cudaStream_t st);
+// the projection along lines with the given tables (every coefficient of an active source is written);
+// the scratch of callers that may run on different streams must not be shared: partial sums
+// (prj_part_bytes), and tickets that are zero before the first call and after every call
+struct LineScratch { void *part; uint32_t *tickets; };
+bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const *tab, LineScratch const &sc, cudaStream_t st);
+bool launch_project_line(DevicePlan &dp, double *apc, double const *x, void const *tab, LineScratch const &sc, cudaStream_t st);
+bool ensure_line_scratch(DevicePlan const &dp, OwnLineScratch &own, size_t elem_bytes, cudaStream_t st, LineScratch &sc);
+inline size_t prj_part_bytes(DevicePlan const &dp, size_t elem_bytes) {
+    size_t const n = dp.prj_line.part_rows*128*elem_bytes;
+    return n < 16 ? 16 : n;
+}
 bool launch_add_line(DevicePlan &dp, float *y, float const *cad, cudaStream_t st);
 bool launch_add_line(DevicePlan &dp, double *y, double const *cad, cudaStream_t st);
 bool prepare_line_kernels32();

@@ -198,6 +198,8 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
     if (!dp.cadd.alloc(std::max<size_t>(16, size_t(dp.ncoeffA)*dp.nCols*128*sizeof(double)))) return false;
     dp.uploaded = true;
     dp.values_dirty = true;
+    // the tables above are made on the legacy stream; the plan may be used on any stream from here on
+    A43G_CUDA_TRY(cudaStreamSynchronize(nullptr));
     return upload_values(hp, dp);
 }
 
@@ -243,6 +245,7 @@ bool build_prj_items(GreenPlan const &hp, DevicePlan &dp) {
     }
     dp.prj_line.count = uint32_t(line.size());
     dp.prj_line.part_rows = rows;
+    dp.prj_line.groups = groups;
     return put(dp.prj_line.items, line) && put(dp.prj_line.tickets, std::vector<uint32_t>(4*size_t(groups), 0u));
 }
 
@@ -304,7 +307,19 @@ bool make_line_table(DevicePlan const &dp, double const *slot_H, DeviceBuffer &t
 }
 
 bool ensure_prj_part(DevicePlan &dp, size_t elem_bytes) {
-    return dp.prj_part.alloc(std::max<size_t>(16, dp.prj_line.part_rows*128*elem_bytes));
+    return dp.prj_part.alloc(prj_part_bytes(dp, elem_bytes));
+}
+
+bool ensure_line_scratch(DevicePlan const &dp, OwnLineScratch &own, size_t elem_bytes, cudaStream_t st, LineScratch &sc) {
+    if (!own.part.alloc(prj_part_bytes(dp, elem_bytes))) return false;
+    if (own.groups < dp.prj_line.groups || !own.tickets.ptr) {
+        size_t const n = std::max<size_t>(16, 4*dp.prj_line.groups*sizeof(uint32_t));
+        if (!own.tickets.alloc(n)) return false;
+        A43G_CUDA_TRY(cudaMemsetAsync(own.tickets.ptr, 0, n, st));
+        own.groups = dp.prj_line.groups;
+    }
+    sc = LineScratch{own.part.ptr, dptr<uint32_t>(own.tickets)};
+    return true;
 }
 
 bool upload_values(GreenPlan const &hp, DevicePlan &dp) {

@@ -253,11 +253,11 @@ bool prepare_project() {
 }
 
 template <typename T, int LMAX>
-void project(DevicePlan &dp, T *apc, T const *x, void const *tab, T *part, cudaStream_t st) {
+void project(DevicePlan &dp, T *apc, T const *x, void const *tab, LineScratch const &sc, cudaStream_t st) {
     using V = typename LaneOf<T>::V;
     sho_project_line_kernel<T, LMAX><<<dim3(dp.prj_line.count, quarters<T>()), kThreads, project_smem<LMAX>(), st>>>(
         apc, x, dp.nCols, dptr<PrjItem>(dp.prj_line.items), dptr<uint4>(dp.prj_rec), static_cast<V const*>(tab),
-        dp.retire ? dptr<uint8_t>(dp.src_active) : nullptr, part, dptr<uint32_t>(dp.prj_line.tickets));
+        dp.retire ? dptr<uint8_t>(dp.src_active) : nullptr, static_cast<T*>(sc.part), sc.tickets);
 }
 
 // ---------------------------------------------------------------- addition
@@ -484,14 +484,13 @@ bool prepare() {
 }
 
 template <typename T>
-bool launch_project(DevicePlan &dp, T *apc, T const *x, void const *tab, cudaStream_t st) {
+bool launch_project(DevicePlan &dp, T *apc, T const *x, void const *tab, LineScratch const &sc, cudaStream_t st) {
     if (0 == dp.prj_line.count) return true;
-    T *part = dptr<T>(dp.prj_part);
     switch (dp.lmax_max | 1) {
-        case 1: project<T, 1>(dp, apc, x, tab, part, st); break;
-        case 3: project<T, 3>(dp, apc, x, tab, part, st); break;
-        case 5: project<T, 5>(dp, apc, x, tab, part, st); break;
-        default: project<T, 7>(dp, apc, x, tab, part, st); break;
+        case 1: project<T, 1>(dp, apc, x, tab, sc, st); break;
+        case 3: project<T, 3>(dp, apc, x, tab, sc, st); break;
+        case 5: project<T, 5>(dp, apc, x, tab, sc, st); break;
+        default: project<T, 7>(dp, apc, x, tab, sc, st); break;
     }
     count_launch();
     A43G_CUDA_TRY(cudaGetLastError());

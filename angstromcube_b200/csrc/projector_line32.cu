@@ -5,8 +5,9 @@ namespace a43g {
 
 bool prepare_line_kernels32() { return line::prepare<float>(); }
 
-bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const *tab, cudaStream_t st) {
-    return line::launch_project<float>(dp, apc, x, tab, st);
+bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const *tab, LineScratch const &sc,
+                         cudaStream_t st) {
+    return line::launch_project<float>(dp, apc, x, tab, sc, st);
 }
 
 bool launch_add_line(DevicePlan &dp, float *y, float const *cad, cudaStream_t st) {

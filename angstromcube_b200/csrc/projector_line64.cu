@@ -5,8 +5,9 @@ namespace a43g {
 
 bool prepare_line_kernels64() { return line::prepare<double>(); }
 
-bool launch_project_line(DevicePlan &dp, double *apc, double const *x, void const *tab, cudaStream_t st) {
-    return line::launch_project<double>(dp, apc, x, tab, st);
+bool launch_project_line(DevicePlan &dp, double *apc, double const *x, void const *tab, LineScratch const &sc,
+                         cudaStream_t st) {
+    return line::launch_project<double>(dp, apc, x, tab, sc, st);
 }
 
 bool launch_add_line(DevicePlan &dp, double *y, double const *cad, cudaStream_t st) {

@@ -135,9 +135,11 @@ int vjp(GreenPlan const &hp, DevicePlan &dp, VjpWorkspace &ws, double const *L, 
         for (DeviceBuffer *b : {&ws.apc, &ws.lA, &ws.gA})
             if (!b->alloc(std::max<size_t>(16, std::max(nI, nA)*sizeof(double)))) return A43G_ERR_MEMORY;
         double *apc = dptr<double>(ws.apc), *lA = dptr<double>(ws.lA), *gA = dptr<double>(ws.gA);
-        double const *H = dptr<double>(dp.slot_H);
-        if (!launch_project_with(dp, apc, L, H, st) || !launch_collect_with(dp, lA, apc, dptr<double>(ws.phase_conj), st)) return A43G_ERR_CUDA;
-        if (!launch_project_with(dp, apc, G, H, st) || !launch_collect_with(dp, gA, apc, dptr<double>(dp.img_phase), st)) return A43G_ERR_CUDA;
+        LineScratch sc;
+        if (!ensure_line_scratch(dp, ws.lines, 8, st, sc)) return A43G_ERR_MEMORY;
+        void const *H = dp.line_tab64.ptr;
+        if (!launch_project_line(dp, apc, L, H, sc, st) || !launch_collect_with(dp, lA, apc, dptr<double>(ws.phase_conj), st)) return A43G_ERR_CUDA;
+        if (!launch_project_line(dp, apc, G, H, sc, st) || !launch_collect_with(dp, gA, apc, dptr<double>(dp.img_phase), st)) return A43G_ERR_CUDA;
         if (dM) {
             if (!ws.dM.alloc(std::max<size_t>(16, nmat*sizeof(double)))) return A43G_ERR_MEMORY;
             if (cudaSuccess != cudaMemsetAsync(ws.dM.ptr, 0, nmat*sizeof(double), st)) { set_error("memset"); return A43G_ERR_CUDA; }
@@ -150,7 +152,12 @@ int vjp(GreenPlan const &hp, DevicePlan &dp, VjpWorkspace &ws, double const *L, 
         }
         if (dR) {
             if (!ws.tables_ready) {
-                for (int d = 0; d < 3; ++d) if (!upload(ws.slot_Hd[d], hp.position_derivative_tables(d), st)) return A43G_ERR_CUDA;
+                for (int d = 0; d < 3; ++d) {
+                    if (!upload(ws.slot_H, hp.position_derivative_tables(d), st) ||
+                        !make_line_table(dp, dptr<double>(ws.slot_H), ws.line_Hd[d], nullptr, st)) return A43G_ERR_CUDA;
+                    // the staging buffer and the host table are reused for the next direction
+                    VJP_TRY(cudaStreamSynchronize(st));
+                }
                 ws.tables_ready = true;
             }
             for (DeviceBuffer *b : {&ws.Mg, &ws.dl, &ws.dg, &ws.Mdg})
@@ -160,9 +167,9 @@ int vjp(GreenPlan const &hp, DevicePlan &dp, VjpWorkspace &ws, double const *L, 
             double *Mg = dptr<double>(ws.Mg), *dl = dptr<double>(ws.dl), *dg = dptr<double>(ws.dg), *Mdg = dptr<double>(ws.Mdg);
             if (!launch_mul_with(dp, Mg, gA, st)) return A43G_ERR_CUDA;
             for (int d = 0; d < 3; ++d) {
-                double const *Hd = dptr<double>(ws.slot_Hd[d]);
-                if (!launch_project_with(dp, apc, L, Hd, st) || !launch_collect_with(dp, dl, apc, dptr<double>(ws.phase_conj), st)) return A43G_ERR_CUDA;
-                if (!launch_project_with(dp, apc, G, Hd, st) || !launch_collect_with(dp, dg, apc, dptr<double>(dp.img_phase), st)) return A43G_ERR_CUDA;
+                void const *Hd = ws.line_Hd[d].ptr;
+                if (!launch_project_line(dp, apc, L, Hd, sc, st) || !launch_collect_with(dp, dl, apc, dptr<double>(ws.phase_conj), st)) return A43G_ERR_CUDA;
+                if (!launch_project_line(dp, apc, G, Hd, sc, st) || !launch_collect_with(dp, dg, apc, dptr<double>(dp.img_phase), st)) return A43G_ERR_CUDA;
                 if (!launch_mul_with(dp, Mdg, dg, st)) return A43G_ERR_CUDA;
                 vjp_dot_kernel<<<dp.nAtoms, 256, 0, st>>>(dptr<double>(ws.dR), dl, Mg, dp.nCols, dptr<uint32_t>(dp.atom_starts), dptr<int8_t>(dp.atom_lmax), d);
                 count_launch();

@@ -11,8 +11,10 @@ struct VjpWorkspace {
     DeviceBuffer apc, lA, gA;                 // image projections, collected projections of L and G
     DeviceBuffer Mg, dl, dg, Mdg;             // position derivatives
     DeviceBuffer phase_conj;                  // conjugated image phases
-    DeviceBuffer slot_Hd[3];                  // projector tables differentiated along x, y, z
-    bool tables_ready = false;                // slot_Hd uploaded (the plan geometry is fixed)
+    DeviceBuffer slot_H;                      // staging of a differentiated table
+    DeviceBuffer line_Hd[3];                  // line tables differentiated along x, y, z
+    bool tables_ready = false;                // line_Hd made (the plan geometry is fixed)
+    OwnLineScratch lines;
 };
 
 // L, G: device FP64 block vectors [nnzb][2][64][64]; dV, dM, dR: host outputs or null
