@@ -725,33 +725,46 @@ sho_broadcast_kernel(T *__restrict__ cad, double const *__restrict__ cadd, uint3
 // The atom-matrix chain in one kernel (collect, multiply, broadcast of the three kernels above),
 // per (atom, source, half of the 64 columns): the coefficients of the atom's images summed with
 // their Bloch phases into shared memory, multiplied by M_A (complex, FP64) and written to every
-// image with the conjugate phase.  Warp g of the four works on rows g, g + 4, ... (M_A's rows are
-// uniform over a warp), lane j on column half*32 + j.  Plans without periodic images take no
-// phases (the reference's direct path).  nSHO <= 56.
-constexpr int kAtomRows = 56;
+// image with the conjugate phase.  M_A is copied to shared memory while the images are summed (read
+// from global memory element by element, every fourth one waited for the L2).  Warp g of the eight
+// works on the rows g, g + 8, ... all at once, lane j on column half*32 + j.  Plans without periodic
+// images take no phases (the reference's direct path).  nSHO <= 56.
+//
+// Measured against rows one after the other on 4 warps with M_A from global memory: 8 atoms, 4
+// sources 98 -> 22 us; 64 atoms, 8 sources 147 -> 84 us; 193 atoms, 32 sources 1188 -> 646 us.
+// What bounds it: the latency of the image loads (two CTAs per SM: 77 KB of shared memory).
+constexpr int kAtomRows = 56, kAtomWarps = 8;
+int atom_smem(int lmax) { int const n = nsho_c(lmax); return 2*n*n*8 + 2*n*32*8; }
 
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(32*kAtomWarps)
 sho_atom_kernel(T *__restrict__ cad, T const *__restrict__ apc, uint32_t nrhs,
                 int8_t const *__restrict__ atom_lmax, uint32_t const *__restrict__ sum_start,
                 uint32_t const *__restrict__ sum_col, uint32_t const *__restrict__ img_starts,
                 double const *__restrict__ img_phase, double const *__restrict__ mats,
                 uint32_t const *__restrict__ mat_off, int use_phase, DyadicPairs const bp)
 {
-    __shared__ double sre[kAtomRows][32], sim[kAtomRows][32];
+    constexpr int RW = kAtomRows/kAtomWarps;          // rows per warp
     constexpr int kImg = 32;                          // images of the atom staged in shared memory
+    extern __shared__ __align__(16) double atom_raw[];
     __shared__ uint32_t simg[kImg];
     __shared__ double sph[kImg][2];
     int const A = blockIdx.x, s = blockIdx.y, half = blockIdx.z;
-    int const j = threadIdx.x & 31, g = threadIdx.x >> 5, col = half*32 + j;
+    int const tid = threadIdx.x, j = tid & 31, g = tid >> 5, col = half*32 + j;
     if (bp.active && !bp.active[s]) return;
     img_phase += (s/bp.nsrc_pair)*bp.img_stride;
     mats += (s/bp.nsrc_pair)*bp.mat_stride;
     int const nc = nsho_c(atom_lmax[A]);
+    double *M = atom_raw;                             // [2][nc][nc]
+    double *x = atom_raw + 2*nc*nc;                   // [nc][2][32]
+    for (int q = tid; q < nc*nc; q += 32*kAtomWarps)  // 2 nc^2 doubles, 16 bytes at a time
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::
+                     "r"(uint32_t(__cvta_generic_to_shared(M + 2*q))), "l"(mats + mat_off[A] + 2*size_t(q)) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
     uint32_t const k0 = sum_start[A], k1 = sum_start[A + 1];
     // the atom's images (their coefficient start and phase) once, instead of a chain of three
     // dependent loads per row and image
-    for (uint32_t k = k0 + threadIdx.x; k < k1 && k < k0 + kImg; k += blockDim.x) {
+    for (uint32_t k = k0 + tid; k < k1 && k < k0 + kImg; k += 32*kAtomWarps) {
         uint32_t const i = sum_col[k];
         simg[k - k0] = img_starts[i];
         sph[k - k0][0] = img_phase[4*i]; sph[k - k0][1] = img_phase[4*i + 1];
@@ -761,42 +774,68 @@ sho_atom_kernel(T *__restrict__ cad, T const *__restrict__ apc, uint32_t nrhs,
         if (k - k0 < uint32_t(kImg)) { start = simg[k - k0]; pr = sph[k - k0][0]; pi = sph[k - k0][1]; }
         else { uint32_t const i = sum_col[k]; start = img_starts[i]; pr = img_phase[4*i]; pi = img_phase[4*i + 1]; }
     };
-    for (int c = g; c < nc; c += 4) {
-        double re = 0, im = 0;
-        for (uint32_t k = k0; k < k1; ++k) {
-            uint32_t start; double pr, pi;
-            image(k, start, pr, pi);
-            T const *src = apc + ((size_t(start) + c)*nrhs + s)*128;
-            double const xr = double(src[col]), xi = double(src[64 + col]);
+    size_t const stride = size_t(nrhs)*128;
+    double re[RW], im[RW];
+#pragma unroll
+    for (int r = 0; r < RW; ++r) re[r] = im[r] = 0;
+#pragma unroll 2
+    for (uint32_t k = k0; k < k1; ++k) {
+        uint32_t start; double pr, pi;
+        image(k, start, pr, pi);
+        T const *src = apc + (size_t(start)*nrhs + s)*128 + col;
+        T xr[RW], xi[RW];
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            int const c = min(g + r*kAtomWarps, nc - 1);   // clamped rows are not stored
+            xr[r] = src[c*stride]; xi[r] = src[c*stride + 64];
+        }
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            double const a = double(xr[r]), b = double(xi[r]);
             if (use_phase) {
-                re += pr*xr - pi*xi;
-                im += pr*xi + pi*xr;
+                re[r] += pr*a - pi*b;
+                im[r] += pr*b + pi*a;
             } else {
-                re += xr; im += xi;
+                re[r] += a; im[r] += b;
             }
         }
-        sre[c][j] = re; sim[c][j] = im;
     }
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+        int const c = g + r*kAtomWarps;
+        if (c < nc) { x[c*64 + j] = re[r]; x[c*64 + 32 + j] = im[r]; }
+        re[r] = im[r] = 0;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    double const *Mr = mats + mat_off[A], *Mi = Mr + nc*nc;
-    for (int r = g; r < nc; r += 4) {
-        double re = 0, im = 0;
-        for (int k = 0; k < nc; ++k) {
-            double const mr = __ldg(Mr + r*nc + k), mi = __ldg(Mi + r*nc + k);
-            double const xr = sre[k][j], xi = sim[k][j];
-            re += mr*xr - mi*xi;
-            im += mr*xi + mi*xr;
+    double const *Mr[RW];
+#pragma unroll
+    for (int r = 0; r < RW; ++r) Mr[r] = M + min(g + r*kAtomWarps, nc - 1)*nc;
+    int const plane = nc*nc;
+#pragma unroll 2
+    for (int k = 0; k < nc; ++k) {
+        double const a = x[k*64 + j], b = x[k*64 + 32 + j];
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            double const mr = Mr[r][k], mi = Mr[r][plane + k];
+            re[r] += mr*a - mi*b;
+            im[r] += mr*b + mi*a;
         }
-        for (uint32_t k = k0; k < k1; ++k) {
-            uint32_t start; double pr, pi;
-            image(k, start, pr, pi);
-            pi = -pi;
-            T *dst = cad + ((size_t(start) + r)*nrhs + s)*128;
+    }
+    for (uint32_t k = k0; k < k1; ++k) {
+        uint32_t start; double pr, pi;
+        image(k, start, pr, pi);
+        pi = -pi;
+        T *dst = cad + (size_t(start)*nrhs + s)*128 + col;
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+            int const c = g + r*kAtomWarps;
+            if (c >= nc) break;                       // uniform over the warp
             if (use_phase) {
-                dst[col] = T(pr*re - pi*im);
-                dst[64 + col] = T(pr*im + pi*re);
+                dst[c*stride] = T(pr*re[r] - pi*im[r]);
+                dst[c*stride + 64] = T(pr*im[r] + pi*re[r]);
             } else {
-                dst[col] = T(re); dst[64 + col] = T(im);
+                dst[c*stride] = T(re[r]); dst[c*stride + 64] = T(im[r]);
             }
         }
     }
@@ -910,6 +949,8 @@ bool prepare_local_kernels() {
     // the pencil kernel's three z-slots are 48 KB of dynamic shared memory beside its static part
     A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
     A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(sho_atom_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, atom_smem(5)));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(sho_atom_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, atom_smem(5)));
     return true;
 }
 
@@ -1011,7 +1052,7 @@ bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, c
     }
     dim3 const ga = row_grid(dp), gm = mul_grid(dp);
     if (dp.lmax_max <= 5 && !dp.atom_chain3) {
-        sho_atom_kernel<T><<<dim3(dp.nAtoms, dp.nCols, 2), 128, 0, st>>>(dptr<T>(dp.cad), dptr<T>(dp.apc), dp.nCols,
+        sho_atom_kernel<T><<<dim3(dp.nAtoms, dp.nCols, 2), 32*kAtomWarps, atom_smem(dp.lmax_max), st>>>(dptr<T>(dp.cad), dptr<T>(dp.apc), dp.nCols,
             dptr<int8_t>(dp.atom_lmax), dptr<uint32_t>(dp.sum_start), dptr<uint32_t>(dp.sum_col),
             dptr<uint32_t>(dp.img_starts), dptr<double>(dp.img_phase), dptr<double>(dp.atom_mat),
             dptr<uint32_t>(dp.atom_mat_off), dp.nAI > dp.nAtoms ? 1 : 0, dyadic_pairs(dp));
