@@ -119,9 +119,8 @@ def vjp(plan, L, G, potential=True, matrices=True, positions=True, stream=0):
       "V": complex [ncells, 64]        dF/dV in cell-cube layout,
       "M": list of complex [nc, nc]    dF/dM_A per plan atom (order of export()["global_atom_ids"]),
       "R": complex [nAtoms, 3]         dF/dR_A (atom positions)."""
-    e = plan.export()
-    nat = len(e["AtomLmax"])
-    ncs = [((int(l) + 1) * (int(l) + 2) * (int(l) + 3)) // 6 for l in e["AtomLmax"]]   # int8 in the export
+    ncs = plan.atom_sizes()
+    nat = len(ncs)
     dV = np.zeros((plan.sizes["ncells"], 64, 2)) if potential else None
     dM = np.zeros(max(1, sum(2 * n * n for n in ncs))) if matrices else None
     dR = np.zeros((max(nat, 1), 3, 2)) if positions else None
@@ -129,15 +128,18 @@ def vjp(plan, L, G, potential=True, matrices=True, positions=True, stream=0):
     check(_lib.lib().a43g_vjp(plan.handle, ptr(L), ptr(G), ptr(dV), ptr(dM), ptr(dR), st), "a43g_vjp")
     out = {}
     if potential:
-        out["V"] = dV[..., 0] + 1j * dV[..., 1]
+        out["V"] = dV.view(np.complex128)[..., 0]        # (re, im) pairs
     if matrices:
         mats, o = [], 0
         for n in ncs:
-            mats.append(dM[o:o + n * n].reshape(n, n) + 1j * dM[o + n * n:o + 2 * n * n].reshape(n, n))
+            m = np.empty((n, n), np.complex128)
+            m.real = dM[o:o + n * n].reshape(n, n)
+            m.imag = dM[o + n * n:o + 2 * n * n].reshape(n, n)
+            mats.append(m)
             o += 2 * n * n
         out["M"] = mats
     if positions:
-        out["R"] = (dR[..., 0] + 1j * dR[..., 1])[:nat]
+        out["R"] = dR.view(np.complex128)[..., 0][:nat]
     return out
 
 
@@ -145,8 +147,7 @@ def get_projection_coefficients(plan, G, stream=0):
     """Atomic density matrices Im <p_i|G|p_j> (green_dyadic::get_projection_coefficients) of a
     CUDA float64 Green function G [nnzb, 2, 64, 64]: a list of [nSHO, nSHO] arrays in the order of
     export()["global_atom_ids"]."""
-    e = plan.export()
-    ns = [((int(l) + 1) * (int(l) + 2) * (int(l) + 3)) // 6 for l in e["AtomLmax"]]
+    ns = plan.atom_sizes()
     out = np.zeros(max(1, sum(n * n for n in ns)))
     st = ctypes.c_void_p(stream if isinstance(stream, int) else stream.cuda_stream)
     check(_lib.lib().a43g_projection_coefficients(plan.handle, ptr(G), ptr(out), st), "a43g_projection_coefficients")

@@ -102,6 +102,14 @@ class ActionPlan:
         a["FD_range"] = np.array([s["FD_range%d" % d] for d in range(3)], np.int32)
         return a
 
+    def atom_sizes(self):
+        """Number of SHO functions of every plan atom (export()["AtomLmax"] without the other arrays)."""
+        lmax = np.zeros(max(self.sizes["nAtoms"], 1), np.int8)
+        e = _lib.PlanExport()
+        e.AtomLmax = lmax.ctypes.data
+        check(_lib.lib().a43g_plan_export(self.handle, ctypes.byref(e)), "a43g_plan_export")
+        return [((int(l) + 1) * (int(l) + 2) * (int(l) + 3)) // 6 for l in lmax[:self.sizes["nAtoms"]]]
+
     def upload(self):
         check(_lib.lib().a43g_plan_upload(self.handle), "a43g_plan_upload")
 
