@@ -241,25 +241,26 @@ local_fused_kernel(T *__restrict__ y, T const *__restrict__ x,
 // Pencil kernel (FP32 and FP64): one CTA per (z-line, group of 16 lanes of columns).  A lane holds 8
 // bytes of columns, one in FP64, two in FP32 (.f32x2 arithmetic); a warp is one z-plane zq, its two
 // halves the planes re and im.  A thread owns the 16 points of its plane: the x- and y-stencils run
-// in registers, the rows of the x- and y-neighbours come straight from global memory (the L2) and
-// are applied as they arrive.  Only the z-stencil reads shared memory, where the previous, current
+// in registers, the rows of the x- and y-neighbours come straight from global memory (the L2), those
+// in x a z-stencil ahead of their use.  Only the z-stencil reads shared memory, where the previous, current
 // and next cube of the line are staged by 16-byte asynchronous copies, [slot][re, im][point][lane]
 // (a half warp reads 128 contiguous bytes); the copy of the cube after the next one starts as soon
 // as the z-stencil is done with the previous cube.  The only couplings of re and im, -i Im(E) x and
 // the Bloch phases of halo cubes, take the other plane's values from the partner lane (lane ^ 16).
 //
-// Measured on the 64-atom cell with 8 sources (32,768 blocks): FP64 1.61 ms (4.3 GB read and written
-// once: 0.66 ms), FP32 0.83 ms.  With the z-successor held in registers a step ahead instead of
-// copied, one FP32 column per lane, and the length of the line found by walking it: 1.80 and 0.89
-// ms.  Three CTAs per SM in FP64 (168 registers) rather than four: at 128 registers too few of the
-// neighbour rows' loads are in flight (1.92 ms).  What bounds it: the latency of those loads, and
-// the 8 shared-memory reads per point of the z-stencil.
+// Measured on the 64-atom cell with 8 sources (32,768 blocks): FP64 1.36 ms (4.3 GB read and written
+// once: 0.66 ms), FP32 0.68 ms; with the x-neighbours' rows loaded after the barrier 1.60 and 0.83
+// ms; with the z-successor also in registers instead of copied, one FP32 column per lane, and the
+// length of the line found by walking it, 1.80 and 0.89 ms.  Three CTAs per SM (168 registers): four
+// leave too few of the rows in flight (FP64 1.92 ms), two too few warps (1.55 ms), and carrying the
+// rows of the y-neighbours and of the next step ahead as well spills (1.67 ms).  What bounds it: the
+// latency of those loads, and the 8 shared-memory reads per point of the z-stencil.
 constexpr int kMaxLine = 128;        // cubes of a line (the host checks)
 constexpr int kPencilThreads = 128;
 constexpr int kPencilSmem = 3*2*64*16*8;          // bytes of the three z-slots
 
 template <typename T>
-__global__ void __launch_bounds__(kPencilThreads, sizeof(T) == 8 ? 3 : 4)
+__global__ void __launch_bounds__(kPencilThreads, 3)
 local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
                     uint32_t const *__restrict__ zstart, int32_t const *__restrict__ zlist,
                     int32_t const *__restrict__ nbr, int32_t const *__restrict__ veff,
@@ -333,6 +334,10 @@ local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
         int32_t const exm = code[k][1], exp_ = code[k][2], eym = code[k][3], eyp = code[k][4], iloc = code[k][5];
         V const *pxm = base(exm), *pxp = base(exp_), *pym = base(eym), *pyp = base(eyp);
         T const *pot = ((iloc < 0) ? zero : Vcell + size_t(iloc)*64) + zq*16;
+        // the rows of the x-neighbours, requested before the z-stencil and its barrier
+        V xm[16], xp[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) { xm[i] = __ldg(pxm + i*S); xp[i] = __ldg(pxp + i*S); }
         V cur[16], acc[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) cur[i] = mine[sc*SLOT + i*16];
@@ -365,7 +370,7 @@ local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
         for (int yy = 0; yy < 4; ++yy) {
             V l[12];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { l[i] = __ldg(pxm + (yy*4 + i)*S); l[4 + i] = cur[yy*4 + i]; l[8 + i] = __ldg(pxp + (yy*4 + i)*S); }
+            for (int i = 0; i < 4; ++i) { l[i] = xm[yy*4 + i]; l[4 + i] = cur[yy*4 + i]; l[8 + i] = xp[yy*4 + i]; }
             if (exm < -1) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) l[i] = phase(l[i], a.ph[0][0][0], a.ph[0][0][1]);
