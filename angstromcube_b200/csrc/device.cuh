@@ -50,6 +50,7 @@ struct AddSegment { uint32_t blk[kSegment]; uint64_t any[kSegment]; uint32_t fir
 // one image near a segment: its first coefficient and basis size, and per cube of the segment the
 // slot (kNoSlot: not near) and the mask; the cubes share the y- and z-tables of yz_slot
 struct AddRecord { uint32_t coeff, lmax, slot[kSegment], yz_slot, pad; uint64_t mask[kSegment]; };
+static_assert(0 == sizeof(AddRecord) % 16, "the kernel copies records 16 bytes at a time");
 
 // scratch of a projection outside the action (its own stream)
 struct OwnLineScratch { DeviceBuffer part, tickets; size_t groups = 0; };

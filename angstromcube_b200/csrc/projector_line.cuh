@@ -262,10 +262,6 @@ void project(DevicePlan &dp, T *apc, T const *x, void const *tab, LineScratch co
 
 // ---------------------------------------------------------------- addition
 
-__device__ __forceinline__ void copy8(void *dst, void const *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" :: "r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
 constexpr int kRecs = 32;             // records of a segment held in shared memory at a time
 constexpr int kStages = 3;            // records whose coefficients and tables are in flight or in use
 
@@ -337,14 +333,14 @@ __device__ __forceinline__ void add_image(V (&acc)[SEG][16], V const *c, V const
 // every cube, a lane 8 bytes of columns.  Per image the coefficients are contracted with the
 // z-functions of the plane (56 multiply-adds at L = 5) and the y-functions of the rows (84) once for
 // the whole segment, then with the x-functions of every cube (96); the sums over all images stay in
-// registers and y is read (staged from the start of the CTA on) and written once.  Coefficients and
+// registers and y is read and written once at the end.  Coefficients and
 // tables of the next two records are in flight while one is applied.
 //
 // Measured on the 64-atom cell with 8 sources, against one contraction per (block, image) pair:
-// FP32 1.91 -> 1.02 ms, FP64 3.86 -> 2.07 ms.  The FP64 pipe is 31 % busy (issue slots 32 %): the
-// point sums take 128 of the 244 registers, which leaves two CTAs per SM, and the warps of a CTA
-// meet at every record.  Segments of 4 cubes against 2: 294 multiply-adds per record for 2 cubes
-// touched on average, instead of 2 x 236.
+// FP32 1.91 -> 0.93 ms, FP64 3.86 -> 1.87 ms (1.02 and 2.07 ms with y staged in shared memory from
+// the start of the CTA on).  The FP64 pipe is about a third busy (issue slots too): the point sums
+// take 128 of the 244 registers, which leaves two CTAs per SM.  Segments of 2 cubes and three CTAs
+// per SM are 2 % slower there, and two records per barrier no faster.
 template <typename T, int LMAX, int SEG>
 __global__ void __launch_bounds__(kThreads, LMAX <= 5 ? 2 : 1)
 sho_add_line_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs, AddSegment const *__restrict__ segs,
@@ -356,8 +352,7 @@ sho_add_line_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs,
     constexpr int S = 64*int(sizeof(T))/8;                      // lanes of 8 bytes per point
     extern __shared__ __align__(16) unsigned char smem_line[];
     V *ring = reinterpret_cast<V*>(smem_line);                  // [kStages][NC + NT]
-    V *ys = ring + kStages*(NC + NT);                           // [SEG*16][kThreads] y of this thread's points
-    AddRecord *rec = reinterpret_cast<AddRecord*>(ys + SEG*16*kThreads);   // [kRecs]
+    AddRecord *rec = reinterpret_cast<AddRecord*>(ring + kStages*(NC + NT));   // [kRecs]
     int const tid = threadIdx.x, zq = tid >> 5, lane = tid & 31, quarter = blockIdx.y;
     AddSegment const *seg = segs + blockIdx.x;
     uint32_t const src = seg->src;
@@ -409,15 +404,6 @@ sho_add_line_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs,
             copy_wait<1>();
             __syncthreads();                                    // record i has landed; record i - 1 is done with
             if (i + 2 < n) stage(i + 2);
-            if (0 == r0 + i) {
-#pragma unroll
-                for (int s = 0; s < SEG; ++s)
-                    if (plane(seg->any[s])) {
-                        V const *p = reinterpret_cast<V const*>(yl + size_t(seg->blk[s])*8192);
-#pragma unroll
-                        for (int k = 0; k < 16; ++k) copy8(ys + (16*s + k)*kThreads + tid, p + k*S);
-                    }
-            }
             copy_commit();
             V const *c = ring + (i % kStages)*(NC + NT) + lane;
             V const *t = ring + (i % kStages)*(NC + NT) + NC;
@@ -432,20 +418,32 @@ sho_add_line_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs,
             }
         }
     }
-    copy_wait<0>();                                             // y of this thread's own points
+    // y: two cubes' reads in flight at a time
+    static_assert(0 == SEG % 2, "cubes are updated in pairs");
 #pragma unroll
-    for (int s = 0; s < SEG; ++s)
-        if (plane(seg->any[s])) {
-            V *p = reinterpret_cast<V*>(yl + size_t(seg->blk[s])*8192);
+    for (int s = 0; s < SEG; s += 2) {
+        V v[2][16];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) p[k*S] = vadd(ys[(16*s + k)*kThreads + tid], acc[s][k]);
-        }
+        for (int h = 0; h < 2; ++h)
+            if (plane(seg->any[s + h])) {
+                V const *p = reinterpret_cast<V const*>(yl + size_t(seg->blk[s + h])*8192);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) v[h][k] = p[k*S];
+            }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (plane(seg->any[s + h])) {
+                V *p = reinterpret_cast<V*>(yl + size_t(seg->blk[s + h])*8192);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) p[k*S] = vadd(v[h][k], acc[s + h][k]);
+            }
+    }
 }
 
 template <int LMAX> constexpr int segment_cubes() { return LMAX <= 5 ? int(kSegment) : int(kSegment)/2; }
 template <int LMAX> constexpr int add_smem() {
     constexpr int SEG = segment_cubes<LMAX>();
-    return (kStages*(nsho_of(LMAX)*32 + (4*SEG + 8)*(LMAX + 1)) + SEG*16*kThreads)*8 + kRecs*int(sizeof(AddRecord));
+    return kStages*(nsho_of(LMAX)*32 + (4*SEG + 8)*(LMAX + 1))*8 + kRecs*int(sizeof(AddRecord));
 }
 
 template <typename T, int LMAX>
