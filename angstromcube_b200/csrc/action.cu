@@ -321,7 +321,7 @@ local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
     V const cy1 = vdup(a.st.c[1][1]), cy2 = vdup(a.st.c[1][2]), cy3 = vdup(a.st.c[1][3]), cy4 = vdup(a.st.c[1][4]);
     V const cz1 = vdup(a.st.c[2][1]), cz2 = vdup(a.st.c[2][2]), cz3 = vdup(a.st.c[2][3]), cz4 = vdup(a.st.c[2][4]);
     V const cx[5] = {V(0), cx1, cx2, cx3, cx4}, cy[5] = {V(0), cy1, cy2, cy3, cy4}, cz[5] = {V(0), cz1, cz2, cz3, cz4};
-    T const shift = (a.st.c[0][0] + a.st.c[1][0] + a.st.c[2][0]) - a.E_re;
+    V const c0 = vdup(a.st.c[0][0] + a.st.c[1][0] + a.st.c[2][0]);
     V const eim = vdup(pl ? -a.E_im : a.E_im);                 // re: + Im(E) im, im: - Im(E) re
     __syncthreads();                                           // code[] complete
     fetch(0, zleft); fetch(1, code[0][0]); fetch(2, code[0][6]);
@@ -344,7 +344,8 @@ local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
         // potential and centre; the other plane of the own points from the partner lane
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-            acc[i] = vfma(vdup(__ldg(pot + i) + shift), cur[i], vmul(eim, __shfl_xor_sync(0xffffffffu, cur[i], 16)));
+            acc[i] = vfma(c0, cur[i], vfma(vdup(__ldg(pot + i) - a.E_re), cur[i],
+                                           vmul(eim, __shfl_xor_sync(0xffffffffu, cur[i], 16))));
         // z-stencil from the three staged cubes
 #pragma unroll
         for (int d = 1; d <= 4; ++d) {

@@ -3,8 +3,8 @@
 // The kernels have a few schedule parameters whose best value depends on the plan (how many
 // blocks, how many atom images per block, how long the z-lines are) and on the GPU:
 //   * prj_chunk   : blocks of one (image, source) list per projection CTA (the cubes-per-CTA
-//                   schedule of the projection: longer chunks amortize the pipeline start and
-//                   the coefficient atomics, shorter ones balance the load)   {12, 24, 40}
+//                   schedule of the projection: longer chunks amortize the start and the
+//                   partial sums, shorter ones balance the load)   {12, 24, 40}
 //   * use_tc      : FP32 projector on the tensor cores (3xTF32) or on the CUDA cores
 // Each parameter is tuned in turn (coordinate descent), every candidate timed with CUDA events
 // on the caller's stream: two untimed applications, then the mean of three.  Scratch vectors
@@ -85,8 +85,8 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
             }
         }
     }
-    std::snprintf(line, sizeof(line), "chosen: projector chunk %u, %s projector\n",
-                  dp.prj_chunk, dp.use_tc ? "tensor-core" : "CUDA-core");
+    std::snprintf(line, sizeof(line), "chosen: projector chunk %u, local %s, %s projector\n",
+                  dp.prj_chunk, dp.local_rows ? "plain rows" : "pencils", dp.use_tc ? "tensor-core" : "CUDA-core");
     report += line;
     A43G_CUDA_TRY(cudaStreamSynchronize(st));
     return true;

@@ -94,7 +94,7 @@ struct DevicePlan {
     DeviceBuffer slot_H32;       // float copy of slot_H for the FP32 kernels
     int table_stride = 0;        // doubles per slot in slot_H
     DeviceBuffer dev_error;      // int: first error code recorded by a kernel (0: none)
-    bool use_tc = true;          // FP32 projector on the tensor cores (else SIMT)
+    bool use_tc = true;          // FP32 projector on the tensor cores (else the CUDA cores)
     struct ImageGroup { uint32_t count = 0; DeviceBuffer images; } img_group[8];  // images by basis size
     // work items of the generic projection kernel by basis size: (image, source, first, last) list
     // positions, each at most 16 blocks

@@ -183,7 +183,7 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
     dp.mat_stride = hp.AtomMatrices.size();
     if (!put(dp.dev_error, std::vector<int32_t>(4, 0))) return false;
     {
-        // FP32 projector: SIMT (default) or the tensor cores ("tc"); the FP64 path is always SIMT
+        // FP32 projector: CUDA cores (default) or the tensor cores ("tc"); FP64 always on the CUDA cores
         char const *e = std::getenv("A43G_PROJECTOR");
         dp.use_tc = (e && 0 == std::strcmp(e, "tc"));
         // local kernel: pencils (default) or "rows" ("plain" in FP32), the kernel of unaligned vectors

@@ -490,7 +490,7 @@ def measure_kernels(plan, stream, out, hbm, bf16, peak_kind):
     tf32_peak = bf16 / 2
     tc = os.environ.get("A43G_PROJECTOR", "") == "tc"
     out["roofline_projector"] = {"kernel": ("sho_project_tc + sho_add_tc (tcgen05 kind::tf32, 3xTF32)" if tc else
-                                            "sho_project_simt + sho_add_simt (FP32 CUDA cores, sum-factorized)")
+                                            "sho_project_line + sho_add_line (FP32 CUDA cores, sum-factorized along lines of cubes)")
                                  + " + atom matrices",
                                  "bound": "tensor", "achieved": flops / t_dyadic / 1e12, "peak": tf32_peak,
                                  "unit": "TFLOP/s", "frac": flops / t_dyadic / 1e12 / tf32_peak,
@@ -644,18 +644,15 @@ def profile_case(a):
                   "projector_ms": t1 * 1e3})
         x = x.double()
         y = torch.empty_like(x)
-        for name, env in (("pencils, addition unrolled", {}), ("rows, addition rolled",
-                                                               {"A43G_LOCAL64": "rows", "A43G_ADD64": "rolled"})):
-            for k in ("A43G_LOCAL64", "A43G_ADD64"):
-                os.environ.pop(k, None)
+        for name, env in (("pencils", {}), ("rows", {"A43G_LOCAL64": "rows"})):
+            os.environ.pop("A43G_LOCAL64", None)
             os.environ.update(env)
             p = plan_for("simt")
             t0 = time_part(_lib, p, 0, _lib.A43G_F64, x, y, 4, stream)
             t1 = time_part(_lib, p, 1, _lib.A43G_F64, x, y, 4, stream)
             emit({"case": "action", "precision": "float64", "kernels": name, "local_ms": t0 * 1e3,
                   "projector_ms": t1 * 1e3})
-        for k in ("A43G_LOCAL64", "A43G_ADD64"):
-            os.environ.pop(k, None)
+        os.environ.pop("A43G_LOCAL64", None)
     else:
         p = plan_for("simt")
         for precision in ("float32", "float64"):
