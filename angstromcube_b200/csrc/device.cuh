@@ -80,15 +80,12 @@ struct DevicePlan {
     DeviceBuffer lists_start[3], lists[3];
     DeviceBuffer zero_block;     // a block of zeros: neighbours that do not exist
     DeviceBuffer colindx;        // uint16 [nnzb]
-    DeviceBuffer rowindx;        // uint32 [nnzb]
-    DeviceBuffer rowCubePos;     // float [nRows][4]
     DeviceBuffer prj_start, prj_col;   // [nCols][nAI+1], concatenated cols
     DeviceBuffer prj_coloff;           // uint64 [nCols]
     DeviceBuffer add_start, add_col;   // [nnzb+1], [nnz]
     DeviceBuffer sum_start, sum_col;   // [nAtoms+1], [nnz]
-    DeviceBuffer img_pos, img_lmax, img_starts, img_phase;
+    DeviceBuffer img_lmax, img_starts, img_phase;
     DeviceBuffer atom_starts, atom_lmax, atom_mat, atom_mat_off;
-    DeviceBuffer grid_dev;       // double [4]: hx, hy, hz, projection radius
     DeviceBuffer subset_dev;     // uint32 [nCols] diagonal block of each source column
     DeviceBuffer slot_H, slot_mask, prj_slot, add_slot;   // projector tables per (image, row)
     DeviceBuffer slot_H32;       // float copy of slot_H for the FP32 kernels

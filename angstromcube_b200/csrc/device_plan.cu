@@ -114,8 +114,6 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
         if (!put(dp.lists[d], hp.kinetic[d].entry)) return false;
     }
     if (!put(dp.colindx, hp.colindx)) return false;
-    if (!put(dp.rowindx, hp.rowindx)) return false;
-    if (!put(dp.rowCubePos, hp.rowCubePos)) return false;
     // dyadic sparsity
     std::vector<uint32_t> ps, pc; std::vector<uint64_t> po;
     for (uint32_t s = 0; s < hp.nCols; ++s) {
@@ -128,11 +126,10 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
     if (!put(dp.prj_start, ps) || !put(dp.prj_col, pc) || !put(dp.prj_coloff, po)) return false;
     if (!put(dp.add_start, hp.SHOadd.start) || !put(dp.add_col, hp.SHOadd.col)) return false;
     if (!put(dp.sum_start, hp.SHOsum.start) || !put(dp.sum_col, hp.SHOsum.col)) return false;
-    if (!put(dp.img_pos, hp.AtomImagePos) || !put(dp.img_lmax, hp.AtomImageLmax)) return false;
+    if (!put(dp.img_lmax, hp.AtomImageLmax)) return false;
     if (!put(dp.img_starts, hp.AtomImageStarts)) return false;
     if (!put(dp.atom_starts, hp.AtomStarts) || !put(dp.atom_lmax, hp.AtomLmax)) return false;
     if (!put(dp.atom_mat_off, hp.AtomMatOffset)) return false;
-    if (!put(dp.grid_dev, std::vector<double>(dp.grid, dp.grid + 4))) return false;
     for (int L = 0; L < 8; ++L) {
         std::vector<uint32_t> imgs;
         for (uint32_t a = 0; a < hp.nAtomImages; ++a) if (hp.AtomImageLmax[a] == L) imgs.push_back(a);
@@ -196,6 +193,10 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
     }
     if (!dp.aac.alloc(std::max<size_t>(16, size_t(dp.ncoeffA)*dp.nCols*128*sizeof(double)))) return false;
     if (!dp.cadd.alloc(std::max<size_t>(16, size_t(dp.ncoeffA)*dp.nCols*128*sizeof(double)))) return false;
+    // coefficient scratch of small plans now (4 MB at most, FP64): the first application of a cell of
+    // 64 blocks would spend 25 times its own time on these allocations
+    if (dp.nAI > 0 && 2*size_t(dp.ncoeffI)*dp.nCols*1024 + prj_part_bytes(dp, 8) <= (size_t(4) << 20) &&
+        (!ensure_dyadic_scratch(dp, 8) || !ensure_prj_part(dp, 8))) return false;
     dp.uploaded = true;
     dp.values_dirty = true;
     // the tables above are made on the legacy stream; the plan may be used on any stream from here on
