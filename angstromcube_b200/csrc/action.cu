@@ -1,10 +1,10 @@
 // The Green-function action y = (H - E S) x on sm_100a.
 //
 //  * local part (potential V - E and the finite-difference kinetic energy) in ONE pass:
-//    local_fused_kernel walks the z-lines of cubes of one source column block, keeps the
-//    z-stencil window in registers and stages the current cube and its four x/y neighbour
-//    cubes in shared memory, so y is written exactly once per block (the reference makes
-//    four passes that re-read and re-write y, include/green_action.hxx:159-167).
+//    local_pencil_kernel walks the z-lines of cubes of one source column block, with the x- and
+//    y-stencils in registers and the z-stencil from three cubes in shared memory, so y is written
+//    exactly once per block (the reference makes four passes that re-read and re-write y,
+//    include/green_action.hxx:159-167).
 //    Plans with a 17-point stencil in some direction use the generic per-direction kernels.
 //  * dyadic part (PAW projectors): projection, atom-matrix multiply, addition
 //    (include/green_dyadic.hxx:856-922), with the image/atom coefficient scratch owned by
@@ -919,7 +919,7 @@ sho_add_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs, uint
 }
 
 // grids of the three-kernel chain: the rows of an atom over the z-index, 4 rows per CTA (a plan of 64
-// atoms and one source would keep 64 CTAs busy with 56 rows each: 239 us against 31 for the collect
+// atoms and one source would keep 64 CTAs busy with 56 rows each: 239 us against 23 for the collect
 // kernel)
 dim3 row_grid(DevicePlan const &dp) { return dim3(dp.nAtoms, dp.nCols, unsigned((nsho_c(std::max(dp.lmax_max, 0)) + 3)/4)); }
 dim3 mul_grid(DevicePlan const &dp) { return dim3(dp.nAtoms, dp.nCols, unsigned((nsho_c(std::max(dp.lmax_max, 0)) + kMulRows - 1)/kMulRows)); }
