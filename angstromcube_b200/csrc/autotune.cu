@@ -47,6 +47,7 @@ template <typename T>
 bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string &report) {
     size_t const n = size_t(dp.nnzb)*8192;
     if (0 == n) return true;
+    if (!readers_done(st)) return false;            // the work items are replaced below
     DeviceBuffer bx, by;
     if (!bx.alloc(n*sizeof(T)) || !by.alloc(n*sizeof(T))) return false;
     A43G_CUDA_TRY(cudaMemsetAsync(bx.ptr, 0x3c, n*sizeof(T), st));   // finite values of moderate size

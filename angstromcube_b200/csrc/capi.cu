@@ -43,7 +43,7 @@ namespace {
 
 int fail(int code, std::string const &msg) { set_error(msg); return code; }
 
-int ensure_device(a43g_plan_t *p) {
+int ensure_device(a43g_plan_t *p, cudaStream_t st) {
     int dev = 0;
     if (cudaSuccess != cudaGetDevice(&dev)) return fail(A43G_ERR_CUDA, "no CUDA device available");
     if (p->device >= 0 && p->device != dev) return fail(A43G_ERR_STATE, "plan was uploaded to another device");
@@ -51,7 +51,7 @@ int ensure_device(a43g_plan_t *p) {
         if (!a43g::upload_plan(p->host, p->dev)) return A43G_ERR_CUDA;
         p->device = dev;
     } else if (p->dev.values_dirty) {
-        if (!a43g::upload_values(p->host, p->dev)) return A43G_ERR_CUDA;
+        if (!a43g::upload_values(p->host, p->dev, st)) return A43G_ERR_CUDA;
     }
     return A43G_OK;
 }
@@ -213,7 +213,7 @@ int a43g_plan_set_kpoint(a43g_plan_t *plan, const double k[3]) {
 int a43g_plan_upload(a43g_plan_t *plan) {
     if (!plan) return fail(A43G_ERR_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(plan->mtx);
-    return ensure_device(plan);
+    return ensure_device(plan, nullptr);
 }
 
 int a43g_action_multiply(a43g_plan_t *plan, void *y, const void *x, const uint16_t *colIndex,
@@ -225,7 +225,7 @@ int a43g_action_multiply(a43g_plan_t *plan, void *y, const void *x, const uint16
     if (nCols != plan->host.nCols) return fail(A43G_ERR_ARGUMENT, "nCols does not match the plan");
     if (!plan->energy_set) return fail(A43G_ERR_STATE, "energy parameter not set (a43g_plan_set_energy)");
     if (y == x) return fail(A43G_ERR_ARGUMENT, "y and x must not alias");
-    int const rc = ensure_device(plan);
+    int const rc = ensure_device(plan, (cudaStream_t)stream);
     if (rc) return rc;
     auto const st = (cudaStream_t)stream;
     bool ok;
@@ -270,7 +270,7 @@ int a43g_plan_autotune(a43g_plan_t *plan, int dtype, void *stream, char *report,
     if (!plan) return fail(A43G_ERR_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(plan->mtx);
     if (!plan->energy_set) return fail(A43G_ERR_STATE, "energy parameter not set (a43g_plan_set_energy)");
-    int const rc = ensure_device(plan);
+    int const rc = ensure_device(plan, (cudaStream_t)stream);
     if (rc) return rc;
     std::string text;
     bool ok;
@@ -289,7 +289,7 @@ int a43g_vjp(a43g_plan_t *plan, const void *L, const void *G, double *dV, double
     if (!plan || !L || !G) return fail(A43G_ERR_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(plan->mtx);
     if (!plan->energy_set) return fail(A43G_ERR_STATE, "energy parameter not set (a43g_plan_set_energy)");
-    int const rc = ensure_device(plan);
+    int const rc = ensure_device(plan, (cudaStream_t)stream);
     if (rc) return rc;
     return a43g::vjp(plan->host, plan->dev, plan->vjpws, (double const*)L, (double const*)G, dV, dM, dR,
                      (cudaStream_t)stream);
@@ -299,7 +299,7 @@ int a43g_action_part(a43g_plan_t *plan, int part, void *y, const void *x, void *
     if (!plan || !y || !x) return fail(A43G_ERR_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(plan->mtx);
     if (!plan->energy_set) return fail(A43G_ERR_STATE, "energy parameter not set (a43g_plan_set_energy)");
-    int const rc = ensure_device(plan);
+    int const rc = ensure_device(plan, (cudaStream_t)stream);
     if (rc) return rc;
     auto const st = (cudaStream_t)stream;
     auto const *ci = a43g::dptr<uint16_t>(plan->dev.colindx);
@@ -332,7 +332,7 @@ int a43g_solve(a43g_plan_t *plan, const a43g_solve_options_t *opts, void *X, dou
     if (!plan || !opts) return fail(A43G_ERR_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(plan->mtx);
     if (!plan->energy_set) return fail(A43G_ERR_STATE, "energy parameter not set (a43g_plan_set_energy)");
-    int const rc = ensure_device(plan);
+    int const rc = ensure_device(plan, (cudaStream_t)stream);
     if (rc) return rc;
     a43g_solve_stats_t local{};
     int const r = a43g::solve(plan->host, plan->dev, plan->solver, *opts, X, rho, stats ? stats : &local,
@@ -346,7 +346,7 @@ int a43g_solve_traced(a43g_plan_t *plan, const a43g_solve_options_t *opts, void 
     if (!plan || !opts || !X_reference || (capacity > 0 && !trace)) return fail(A43G_ERR_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(plan->mtx);
     if (!plan->energy_set) return fail(A43G_ERR_STATE, "energy parameter not set (a43g_plan_set_energy)");
-    int const rc = ensure_device(plan);
+    int const rc = ensure_device(plan, (cudaStream_t)stream);
     if (rc) return rc;
     a43g_solve_stats_t local{};
     a43g::SolveTrace tr;
@@ -368,7 +368,7 @@ int a43g_solve_batched(a43g_plan_t *plan, const a43g_solve_options_t *opts, int3
         return fail(A43G_ERR_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(plan->mtx);
     if (!plan->matrices_set && plan->host.nAtoms > 0) return fail(A43G_ERR_STATE, "atom matrices not set");
-    int const rc = ensure_device(plan);
+    int const rc = ensure_device(plan, (cudaStream_t)stream);
     if (rc) return rc;
     return a43g::solve_batched(plan->host, plan->dev, plan->batch, *opts, n, energies, kpoints, dVol,
                                rho, stats, (cudaStream_t)stream);
@@ -378,7 +378,7 @@ int a43g_projection_coefficients(a43g_plan_t *plan, const void *G, double *out, 
     if (!plan || !G || !out) return fail(A43G_ERR_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lock(plan->mtx);
     if (!plan->energy_set) return fail(A43G_ERR_STATE, "energy parameter not set (a43g_plan_set_energy)");
-    int const rc = ensure_device(plan);
+    int const rc = ensure_device(plan, (cudaStream_t)stream);
     if (rc) return rc;
     return a43g::projection_coefficients(plan->host, plan->dev, plan->density, (double const*)G, out,
                                          (cudaStream_t)stream);

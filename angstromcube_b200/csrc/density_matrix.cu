@@ -101,6 +101,7 @@ int projection_coefficients(GreenPlan const &hp, DevicePlan &dp, DensityWorkspac
             set_error("upload of the source-cube projector tables");
             return A43G_ERR_CUDA;
         }
+        if (!uploads_landed()) return A43G_ERR_CUDA;
         ws.ready = true;
     }
     if (!ws.apc.alloc(std::max<size_t>(16, nI*8)) || !ws.aac.alloc(std::max<size_t>(16, nA*8))) return A43G_ERR_MEMORY;

@@ -130,8 +130,14 @@ bool prepare_tc_kernels();
 // kernel launch counter: n launches at once (replays of a captured graph)
 void count_launches(uint64_t n);
 uint64_t launches_so_far();
-bool upload_values(GreenPlan const &hp, DevicePlan &dp);
-// projection work items (image, source, up to dp.prj_chunk consecutive blocks of its list)
+// potential, matrices, phases and energies; earlier calls on st are waited for before they are replaced
+bool upload_values(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st);
+// copies of host arrays made on the legacy stream have reached the device: kernels of any stream may
+// read them.  Kernels launched on st have finished: arrays that they read may be replaced.
+bool uploads_landed();
+bool readers_done(cudaStream_t st);
+// projection work items (image, source, up to dp.prj_chunk consecutive blocks of its list); no kernel
+// that reads the present ones may be running (readers_done)
 bool build_prj_items(GreenPlan const &hp, DevicePlan &dp);
 // a table [slot][order][dir][point] of the plan's slots in the layout of the line kernels
 bool make_line_table(DevicePlan const &dp, double const *slot_H, DeviceBuffer &t64, DeviceBuffer *t32, cudaStream_t st);

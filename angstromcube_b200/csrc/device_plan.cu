@@ -79,6 +79,23 @@ bool build_add_segments(GreenPlan const &hp, DevicePlan &dp);
 
 } // namespace
 
+// A copy from pageable memory may return while its last piece is still on the way, and the kernels of
+// a non-blocking stream are not ordered behind the legacy stream that it runs on.
+bool uploads_landed() {
+    A43G_CUDA_TRY(cudaStreamSynchronize(nullptr));
+    return true;
+}
+
+// The legacy stream does not wait for a non-blocking stream either: arrays that kernels launched on st
+// may still read are replaced only when they are done.  A stream under capture has nothing running.
+bool readers_done(cudaStream_t st) {
+    if (!st) return true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    A43G_CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+    if (cudaStreamCaptureStatusNone == cs) A43G_CUDA_TRY(cudaStreamSynchronize(st));
+    return true;
+}
+
 bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
     if (!prepare_line_kernels32() || !prepare_line_kernels64() || !prepare_tc_kernels() || !prepare_local_kernels()) return false;
     dp.nnzb = uint32_t(hp.nnzb()); dp.nRows = hp.nRows; dp.nCols = hp.nCols;
@@ -199,9 +216,7 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
         (!ensure_dyadic_scratch(dp, 8) || !ensure_prj_part(dp, 8))) return false;
     dp.uploaded = true;
     dp.values_dirty = true;
-    // the tables above are made on the legacy stream; the plan may be used on any stream from here on
-    A43G_CUDA_TRY(cudaStreamSynchronize(nullptr));
-    return upload_values(hp, dp);
+    return upload_values(hp, dp, nullptr);          // waits for the legacy stream: the tables above too
 }
 
 bool build_prj_items(GreenPlan const &hp, DevicePlan &dp) {
@@ -247,7 +262,8 @@ bool build_prj_items(GreenPlan const &hp, DevicePlan &dp) {
     dp.prj_line.count = uint32_t(line.size());
     dp.prj_line.part_rows = rows;
     dp.prj_line.groups = groups;
-    return put(dp.prj_line.items, line) && put(dp.prj_line.tickets, std::vector<uint32_t>(4*size_t(groups), 0u));
+    return put(dp.prj_line.items, line) && put(dp.prj_line.tickets, std::vector<uint32_t>(4*size_t(groups), 0u)) &&
+           uploads_landed();
 }
 
 namespace {
@@ -323,7 +339,8 @@ bool ensure_line_scratch(DevicePlan const &dp, OwnLineScratch &own, size_t elem_
     return true;
 }
 
-bool upload_values(GreenPlan const &hp, DevicePlan &dp) {
+bool upload_values(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st) {
+    if (!readers_done(st)) return false;
     if (!put(dp.Vcell64, hp.Vcell)) return false;
     std::vector<float> v32(hp.Vcell.begin(), hp.Vcell.end());
     if (!put(dp.Vcell32, v32)) return false;
@@ -345,6 +362,7 @@ bool upload_values(GreenPlan const &hp, DevicePlan &dp) {
     }
     std::memcpy(dp.phase, hp.phase, sizeof(dp.phase));
     dp.E_re = hp.E_re; dp.E_im = hp.E_im;
+    if (!uploads_landed()) return false;            // the values may be used on any stream from here on
     dp.values_dirty = false;
     return true;
 }

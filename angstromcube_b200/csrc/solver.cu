@@ -1536,7 +1536,7 @@ int solve_batched(GreenPlan &hp, DevicePlan &dp, BatchCache &bc, a43g_solve_opti
             auto const err = bc.host.set_pair(p, energies[2*i], energies[2*i + 1], dVol, kpoints + 3*size_t(i));
             if (!err.empty()) { set_error(err); return A43G_ERR_ARGUMENT; }
         }
-        if (!upload_values(bc.host, *bc.dev)) return A43G_ERR_CUDA;
+        if (!upload_values(bc.host, *bc.dev, st)) return A43G_ERR_CUDA;
         a43g_solve_stats_t ws_stats{};
         SourceStats per;
         per.live_sources = live*nsrc;

@@ -139,7 +139,10 @@ int a43g_plan_set_atom_matrices(a43g_plan_t *plan, const double *mats, const int
 int a43g_plan_set_energy(a43g_plan_t *plan, double E_re, double E_im, double dVol);
 /* replaces green_function::update_phases (src/green_function.cxx:218-251); k in units of 2 pi/cell */
 int a43g_plan_set_kpoint(a43g_plan_t *plan, const double k[3]);
-/* copies plan, potential and matrices to the device (done implicitly by the calls below) */
+/* copies plan, potential and matrices to the device (done implicitly by the calls below) and returns
+ * when they are there, for calls on any stream.  Values that changed replace the old ones on the device:
+ * the calls below first wait for earlier work on their own stream, a43g_plan_upload for the legacy
+ * stream; calls of this plan in flight on other (non-blocking) streams must have finished. */
 int a43g_plan_upload(a43g_plan_t *plan);
 
 /* ---- the operator: replaces green_action::action_t<real_t,2,1,64>::multiply

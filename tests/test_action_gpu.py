@@ -240,6 +240,52 @@ def test_action_rejects_bad_sizes():
         op.multiply(x, x, ci, p.nnzb, p.nCols)
 
 
+def test_values_change_behind_calls_in_flight():
+    """On a non-blocking stream, calls that are still queued keep the energy, phases and matrices they
+    were made with, and the next call sees the new ones; so do calls before and after the autotuner,
+    which replaces the projection's work items."""
+    w = workloads.make("periodic8_8atoms_s2x2x1")
+    p = gf.construct_Green_function(w.geometry)
+    gf.update_potential(p, w.Vcell, w.mats, w.offsets, layout="cells")
+    ci = torch.from_numpy(p.export()["colindx"].astype(np.int16)).cuda()
+    x = torch.randn((p.nnzb, 2, 64, 64), device="cuda", dtype=torch.float64)
+    op = green_action.action_t(p, "float64")
+    settings = [(complex(-0.2, 0.1), (0.0, 0.0, 0.0)), (complex(0.4, 0.3), (0.1, 0.2, -0.15)), (complex(-0.7, 0.01), (0.3, 0.0, 0.2))]
+
+    def set_values(E, k):
+        gf.update_energy_parameter(p, E, w.dVol)
+        gf.update_phases(p, k)
+
+    ref = []
+    for E, k in settings:
+        set_values(E, k)
+        y = torch.empty_like(x)
+        op.multiply(y, x, ci, p.nnzb, p.nCols)
+        torch.cuda.synchronize()
+        ref.append(y)
+    assert not torch.equal(ref[0], ref[1])
+    s = torch.cuda.Stream()
+    out = [torch.empty_like(x) for _ in settings]
+    busy = torch.empty_like(x)
+    torch.cuda.synchronize()
+    for (E, k), y in zip(settings, out):
+        set_values(E, k)
+        for _ in range(10):                                   # some milliseconds of queued work
+            op.multiply(busy, x, ci, p.nnzb, p.nCols, stream=s)
+        op.multiply(y, x, ci, p.nnzb, p.nCols, stream=s)
+    torch.cuda.synchronize()
+    for y, r in zip(out, ref):
+        assert torch.equal(y, r)
+    for _ in range(10):
+        op.multiply(busy, x, ci, p.nnzb, p.nCols, stream=s)
+    op.multiply(out[0], x, ci, p.nnzb, p.nCols, stream=s)
+    green_action.autotune(p, "float64", stream=s)
+    op.multiply(out[1], x, ci, p.nnzb, p.nCols, stream=s)
+    torch.cuda.synchronize()
+    assert torch.equal(out[0], ref[-1])
+    assert rel_err(out[1].cpu().numpy(), ref[-1].cpu().numpy()) < FP64_TOL
+
+
 @pytest.mark.parametrize("name", ["wrap8", "peri_xy_wrap_z"])
 def test_autotune_keeps_parity(name):
     """The autotuner only changes the schedule: after it the FP32 and FP64 actions still match
