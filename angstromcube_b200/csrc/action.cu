@@ -259,7 +259,35 @@ constexpr int kMaxLine = 128;        // cubes of a line (the host checks)
 constexpr int kPencilThreads = 128;
 constexpr int kPencilSmem = 3*2*64*16*8;          // bytes of the three z-slots
 
-template <typename T>
+// a lane's 8 bytes of global memory on an A-byte boundary
+template <int A> __device__ __forceinline__ double lane_load(double const *p) { return __ldg(p); }
+template <int A> __device__ __forceinline__ unsigned long long lane_load(unsigned long long const *p) {
+    if (A >= 8) return __ldg(p);
+    float const *f = reinterpret_cast<float const*>(p);
+    float const a = __ldg(f), b = __ldg(f + 1);
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+template <int A> __device__ __forceinline__ void lane_store(double *p, double v) { *p = v; }
+template <int A> __device__ __forceinline__ void lane_store(unsigned long long *p, unsigned long long v) {
+    if (A >= 8) { *p = v; return; }
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    float *f = reinterpret_cast<float*>(p);
+    f[0] = a; f[1] = b;
+}
+// asynchronous copy of A = 4, 8 or 16 bytes to shared memory (only 16 can pass the L1 by)
+template <int A> __device__ __forceinline__ void copy_async(void *dst, void const *src) {
+    uint32_t const d = uint32_t(__cvta_generic_to_shared(dst));
+    if (16 == A) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" :: "r"(d), "l"(src), "n"(A) : "memory");
+}
+
+// A: the boundary in bytes that x and y lie on (16, 8 or 4); off 16 bytes the copies are as small as A, and
+// two loads and stores make a lane on 4.  On the cell above FP64 takes 1.67 ms on 8 bytes, FP32 0.88 ms on
+// 8 and 0.95 ms on 4; the rows kernel takes 3.56 and 1.49 ms.
+template <typename T, int A>
 __global__ void __launch_bounds__(kPencilThreads, 3)
 local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
                     uint32_t const *__restrict__ zstart, int32_t const *__restrict__ zlist,
@@ -293,11 +321,11 @@ local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
             for (int i = 0; i < 16; ++i) mine[slot*SLOT + i*16] = V(0);
         } else {
             T const *src = x + size_t(nbr_block(e))*kBlockReals + group*16*W;
+            constexpr int P = 128/A, E = A/int(sizeof(T));     // pieces of a row of 128 bytes, elements of a piece
 #pragma unroll
-            for (int q = 0; q < 2*64*8/kPencilThreads; ++q) {
-                int const c = q*kPencilThreads + tid, row = c >> 3, part = c & 7;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::
-                             "r"(uint32_t(__cvta_generic_to_shared(dst + row*16 + 2*part))), "l"(src + row*64 + part*2*W) : "memory");
+            for (int q = 0; q < 2*64*P/kPencilThreads; ++q) {
+                int const c = q*kPencilThreads + tid, row = c/P, part = c % P;
+                copy_async<A>(reinterpret_cast<T*>(dst + row*16) + part*E, src + row*64 + part*E);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -337,7 +365,7 @@ local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
         // the rows of the x-neighbours, requested before the z-stencil and its barrier
         V xm[16], xp[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) { xm[i] = __ldg(pxm + i*S); xp[i] = __ldg(pxp + i*S); }
+        for (int i = 0; i < 16; ++i) { xm[i] = lane_load<A>(pxm + i*S); xp[i] = lane_load<A>(pxp + i*S); }
         V cur[16], acc[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) cur[i] = mine[sc*SLOT + i*16];
@@ -390,7 +418,7 @@ local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
         for (int yo = 0; yo < 4; ++yo) {
             V ym[4], yp[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { ym[i] = __ldg(pym + (yo*4 + i)*S); yp[i] = __ldg(pyp + (yo*4 + i)*S); }
+            for (int i = 0; i < 4; ++i) { ym[i] = lane_load<A>(pym + (yo*4 + i)*S); yp[i] = lane_load<A>(pyp + (yo*4 + i)*S); }
             if (eym < -1) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) ym[i] = phase(ym[i], a.ph[1][0][0], a.ph[1][0][1]);
@@ -410,7 +438,7 @@ local_pencil_kernel(T *__restrict__ y, T const *__restrict__ x,
         }
         V *yb = reinterpret_cast<V*>(y + size_t(code[k][0])*kBlockReals + lo) + zq*16*S;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) yb[i*S] = acc[i];
+        for (int i = 0; i < 16; ++i) lane_store<A>(yb + i*S, acc[i]);
         if (k + 1 < n) {
             land();                                            // the cube after the next one
             if (code[k + 1][6] < -1) { turn(sp, a.ph[2][1]); __syncthreads(); }
@@ -953,8 +981,11 @@ void launch_project_L(DevicePlan &dp, T const *x, cudaStream_t st) {
 
 bool prepare_local_kernels() {
     // the pencil kernel's three z-slots are 48 KB of dynamic shared memory beside its static part
-    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
-    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<float, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<double, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
+    A43G_CUDA_TRY(cudaFuncSetAttribute(local_pencil_kernel<double, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPencilSmem));
     A43G_CUDA_TRY(cudaFuncSetAttribute(sho_atom_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, atom_smem(5)));
     A43G_CUDA_TRY(cudaFuncSetAttribute(sho_atom_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, atom_smem(5)));
     return true;
@@ -983,11 +1014,12 @@ bool launch_local(DevicePlan &dp, T *y, T const *x, cudaStream_t st) {
     if (dp.fused_local) {
         constexpr int S = (sizeof(T) == 8) ? 8 : 16;
         unsigned const nblk = dp.nlists[2]*(64/S);
-        // pencils copy 16 bytes at a time and hold the codes of a line; the rows kernel takes the
-        // other calls
-        bool const pencils = !dp.local_rows && dp.max_zline <= kMaxLine && vectors_aligned16(x, y);
+        // the pencils hold the codes of a line; the rows kernel takes longer lines
+        bool const pencils = !dp.local_rows && dp.max_zline <= kMaxLine;
         if (nblk && pencils) {
-            local_pencil_kernel<T><<<dp.nlists[2]*(unsigned(sizeof(T))/2), kPencilThreads, kPencilSmem, st>>>(y, x,
+            auto *kernel = vectors_aligned(x, y, 16) ? local_pencil_kernel<T, 16> :
+                           vectors_aligned(x, y, 8) ? local_pencil_kernel<T, 8> : local_pencil_kernel<T, int(sizeof(T))>;
+            kernel<<<dp.nlists[2]*(unsigned(sizeof(T))/2), kPencilThreads, kPencilSmem, st>>>(y, x,
                 dptr<uint32_t>(dp.lists_start[2]), dptr<int32_t>(dp.lists[2]), dptr<int32_t>(dp.nbr),
                 dptr<int32_t>(dp.veff_index), vcell<T>(dp), dptr<T>(dp.zero_block), a);
             count_launch();
@@ -1038,10 +1070,11 @@ template <typename T>
 bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, cudaStream_t st) {
     if (dp.nAI < 1 || dp.nCols < 1) return true;
     if (!ensure_dyadic_scratch(dp, sizeof(T))) return false;
-    // both FP32 projector paths stage x with 16-byte loads; other x take the generic kernels
-    bool const aligned16 = 0 == (reinterpret_cast<uintptr_t>(x) & 15u);
+    // the tensor-core projection stages x with 16-byte copies; the line kernels take 8-byte lanes of x and
+    // y, and vectors on 16 bytes; other vectors take the generic kernels
+    bool const aligned16 = vectors_aligned(x, x, 16);
     bool const tc = (sizeof(T) == 4) && dp.use_tc && aligned16 && tc_projector_supported(dp);
-    bool const lines = !tc && vectors_aligned16(x, y);
+    bool const lines = !tc && vectors_aligned(x, y, 16);
     if (tc) {
         if (!launch_project_tc(dp, (float const*)x, st)) return false;
     } else if (lines) {

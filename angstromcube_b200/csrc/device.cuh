@@ -178,10 +178,9 @@ bool tc_projector_supported(DevicePlan const &dp);
 bool launch_project_tc(DevicePlan &dp, float const *x, cudaStream_t st);
 bool launch_add_tc(DevicePlan &dp, float *y, uint16_t const *colIndex, cudaStream_t st);
 
-// vectors that the kernels on 8-byte lanes with 16-byte copies take (local pencils; projection and
-// addition along lines of cubes, projector_line.cuh)
-inline bool vectors_aligned16(void const *x, void const *y) {
-    return 0 == ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u);
+// both vectors lie on a boundary of `bytes` (a power of two)
+inline bool vectors_aligned(void const *x, void const *y, unsigned bytes) {
+    return 0 == ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & uintptr_t(bytes - 1));
 }
 // the projection along lines with the given tables (every coefficient of an active source is written);
 // the scratch of callers that may run on different streams must not be shared: partial sums

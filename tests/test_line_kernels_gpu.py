@@ -11,7 +11,7 @@ import pytest
 
 import oracle
 from helpers import geometry, inputs_for, product_plan, rel_err
-from angstromcube_b200 import green_action
+from angstromcube_b200 import _lib, green_action
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -67,9 +67,30 @@ def test_action_at_the_edges(name, dtype):
 
 @pytest.mark.parametrize("dtype", sorted(TOL))
 def test_vectors_off_the_16_byte_boundary(dtype):
-    """One element further, x and y take the kernels without 16-byte copies."""
+    """One element further, x and y take the projector kernels without 16-byte copies."""
     p, x, ref = plan_and_inputs(GEOMETRIES["mixed_to_5"]())
     assert rel_err(apply(p, x, dtype, offset=1), ref) < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype,xo,yo", [("float64", 1, 0), ("float64", 0, 1), ("float64", 1, 1), ("float32", 2, 0),
+                                         ("float32", 0, 2), ("float32", 1, 0), ("float32", 0, 1), ("float32", 3, 2)])
+@pytest.mark.parametrize("name", ["mixed_to_5", "numax1"])
+def test_pencils_off_the_16_byte_boundary(name, dtype, xo, yo):
+    """The local part of x and y on any element is the pencils': the same sums in the same order as
+    on 16 bytes (the rows kernel adds in another order).  A cell with a boundary of every kind and
+    phases, and one whose lines of cubes are their own neighbours."""
+    p, x_np, _ = plan_and_inputs(GEOMETRIES[name]())
+    t = getattr(torch, dtype)
+    y = []
+    for a, b in ((0, 0), (xo, yo)):
+        xs, ys = (torch.full((x_np.size + o + 4,), 7.0, dtype=t, device="cuda") for o in (a, b))
+        xs[a:a + x_np.size] = torch.from_numpy(x_np.ravel()).to(t)
+        _lib.check(_lib.lib().a43g_action_part(p.handle, 0, ys[b:].data_ptr(), xs[a:].data_ptr(), None,
+                                               green_action.action_t(p, dtype).dtype), "local part")
+        torch.cuda.synchronize()
+        y.append(ys[b:b + x_np.size])
+        assert (ys[:b] == 7).all() and (ys[b + x_np.size:] == 7).all()
+    assert torch.equal(y[0], y[1])
 
 
 @pytest.mark.parametrize("dtype", sorted(TOL))
