@@ -193,8 +193,8 @@ inline size_t prj_part_bytes(DevicePlan const &dp, size_t elem_bytes) {
     size_t const n = dp.prj_line.part_rows*128*elem_bytes;
     return n < 16 ? 16 : n;
 }
-bool launch_add_line(DevicePlan &dp, float *y, float const *cad, cudaStream_t st);
-bool launch_add_line(DevicePlan &dp, double *y, double const *cad, cudaStream_t st);
+bool launch_add_line(DevicePlan &dp, float *y, float const *cad, uint16_t const *colIndex, cudaStream_t st);
+bool launch_add_line(DevicePlan &dp, double *y, double const *cad, uint16_t const *colIndex, cudaStream_t st);
 bool prepare_line_kernels32();
 bool prepare_line_kernels64();
 

@@ -327,6 +327,48 @@ __device__ __forceinline__ void add_image(V (&acc)[SEG][16], V const *c, V const
     }
 }
 
+// a segment whose blocks the caller's colIndex gives to other columns than the plan's: every cube by
+// itself, coefficients and tables read in place (a call that no solver makes).  Kept out of the loop over
+// images: masks by column in there cost 2 to 3 % of the dyadic part of the 64-atom cell, this 0.5 % or less
+template <typename T, int LP, int SEG>
+__device__ __noinline__ void add_by_columns(T *yl, T const *cq, uint32_t nrhs, uint16_t const *colIndex, AddSegment const *seg,
+                                            AddRecord const *recs, typename LaneOf<T>::V const *tab, int zq) {
+    using V = typename LaneOf<T>::V;
+    constexpr int S = 64*int(sizeof(T))/8;
+    for (int s = 0; s < SEG; ++s) {
+        if (!(uint32_t(seg->any[s] >> (16*zq)) & 0xffffu)) continue;
+        T const *cs = cq + size_t(colIndex[seg->blk[s]])*128;
+        V acc[16];
+#pragma unroll
+        for (int p = 0; p < 16; ++p) acc[p] = V(0);
+        for (uint32_t i = 0; i < seg->count; ++i) {
+            AddRecord const &r = recs[i];
+            uint32_t const m = uint32_t(r.mask[s] >> (16*zq)) & 0xffffu;
+            if (!m) continue;
+            int const L = int(r.lmax);
+            V const *hx = tab + size_t(r.slot[s])*12*LP, *hy = hx + 4*LP, *hz = hx + (8 + zq)*LP;
+            T const *c = cs + size_t(r.coeff)*nrhs*128;
+            V f[16];
+#pragma unroll
+            for (int p = 0; p < 16; ++p) f[p] = V(0);
+            for (int iz = 0; iz <= L; ++iz)
+                for (int iy = 0; iy <= L - iz; ++iy) {
+                    V ax[4] = {V(0), V(0), V(0), V(0)};
+                    for (int ix = 0; ix <= L - iz - iy; ++ix, c += size_t(nrhs)*128)
+#pragma unroll
+                        for (int xx = 0; xx < 4; ++xx) ax[xx] = vfma(*reinterpret_cast<V const*>(c), hx[xx*LP + ix], ax[xx]);
+#pragma unroll
+                    for (int p = 0; p < 16; ++p) f[p] = vfma(vmul(hy[(p >> 2)*LP + iy], hz[iz]), ax[p & 3], f[p]);
+                }
+#pragma unroll
+            for (int p = 0; p < 16; ++p) if ((m >> p) & 1u) acc[p] = vadd(acc[p], f[p]);
+        }
+        V *yb = reinterpret_cast<V*>(yl + size_t(seg->blk[s])*8192);
+#pragma unroll
+        for (int p = 0; p < 16; ++p) yb[p*S] = vadd(yb[p*S], acc[p]);
+    }
+}
+
 // y += the projector functions of all images times their coefficients (include/green_dyadic.hxx:
 // 325-518).  CTA = (segment, quarter of the columns): a segment is up to SEG cubes of one x-line of
 // a source that have images, with one record per image near any of them.  Warp z owns plane z of
@@ -343,9 +385,9 @@ __device__ __forceinline__ void add_image(V (&acc)[SEG][16], V const *c, V const
 // per SM are 2 % slower there, and two records per barrier no faster.
 template <typename T, int LMAX, int SEG>
 __global__ void __launch_bounds__(kThreads, LMAX <= 5 ? 2 : 1)
-sho_add_line_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs, AddSegment const *__restrict__ segs,
-                    AddRecord const *__restrict__ recs, typename LaneOf<T>::V const *__restrict__ tab,
-                    uint8_t const *__restrict__ active)
+sho_add_line_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs, uint16_t const *__restrict__ colIndex,
+                    AddSegment const *__restrict__ segs, AddRecord const *__restrict__ recs,
+                    typename LaneOf<T>::V const *__restrict__ tab, uint8_t const *__restrict__ active)
 {
     using V = typename LaneOf<T>::V;
     constexpr int LP = LMAX + 1, TS = 12*LP, NT = (4*SEG + 8)*LP, NC = nsho_of(LMAX)*32;
@@ -418,7 +460,7 @@ sho_add_line_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs,
             }
         }
     }
-    // y: two cubes' reads in flight at a time
+    // y: two cubes' reads in flight at a time, and beside the first ones the caller's columns
     static_assert(0 == SEG % 2, "cubes are updated in pairs");
 #pragma unroll
     for (int s = 0; s < SEG; s += 2) {
@@ -430,6 +472,15 @@ sho_add_line_kernel(T *__restrict__ y, T const *__restrict__ cad, uint32_t nrhs,
 #pragma unroll
                 for (int k = 0; k < 16; ++k) v[h][k] = p[k*S];
             }
+        if (0 == s) {
+            bool other = false;
+#pragma unroll
+            for (int i = 0; i < SEG; ++i) other |= seg->any[i] && colIndex[seg->blk[i]] != src;
+            if (other) {                                        // uniform: the sums are of other columns
+                add_by_columns<T, LP, SEG>(yl, cad + row_lane<T>(quarter, lane), nrhs, colIndex, seg, mine, tab, zq);
+                return;
+            }
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h)
             if (plane(seg->any[s + h])) {
@@ -454,21 +505,21 @@ bool prepare_add() {
 }
 
 template <typename T, int LMAX>
-void add(DevicePlan &dp, T *y, T const *cad, void const *tab, cudaStream_t st) {
+void add(DevicePlan &dp, T *y, T const *cad, uint16_t const *colIndex, void const *tab, cudaStream_t st) {
     using V = typename LaneOf<T>::V;
     sho_add_line_kernel<T, LMAX, segment_cubes<LMAX>()><<<dim3(dp.add_segments, quarters<T>()), kThreads, add_smem<LMAX>(), st>>>(
-        y, cad, dp.nCols, dptr<AddSegment>(dp.add_seg), dptr<AddRecord>(dp.add_rec), static_cast<V const*>(tab),
-        dp.retire ? dptr<uint8_t>(dp.src_active) : nullptr);
+        y, cad, dp.nCols, colIndex, dptr<AddSegment>(dp.add_seg), dptr<AddRecord>(dp.add_rec),
+        static_cast<V const*>(tab), dp.retire ? dptr<uint8_t>(dp.src_active) : nullptr);
 }
 
 template <typename T>
-bool launch_add(DevicePlan &dp, T *y, T const *cad, void const *tab, cudaStream_t st) {
+bool launch_add(DevicePlan &dp, T *y, T const *cad, uint16_t const *colIndex, void const *tab, cudaStream_t st) {
     if (0 == dp.add_segments) return true;
     switch (dp.lmax_max | 1) {
-        case 1: add<T, 1>(dp, y, cad, tab, st); break;
-        case 3: add<T, 3>(dp, y, cad, tab, st); break;
-        case 5: add<T, 5>(dp, y, cad, tab, st); break;
-        default: add<T, 7>(dp, y, cad, tab, st); break;
+        case 1: add<T, 1>(dp, y, cad, colIndex, tab, st); break;
+        case 3: add<T, 3>(dp, y, cad, colIndex, tab, st); break;
+        case 5: add<T, 5>(dp, y, cad, colIndex, tab, st); break;
+        default: add<T, 7>(dp, y, cad, colIndex, tab, st); break;
     }
     count_launch();
     A43G_CUDA_TRY(cudaGetLastError());

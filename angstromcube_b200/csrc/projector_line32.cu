@@ -10,8 +10,8 @@ bool launch_project_line(DevicePlan &dp, float *apc, float const *x, void const 
     return line::launch_project<float>(dp, apc, x, tab, sc, st);
 }
 
-bool launch_add_line(DevicePlan &dp, float *y, float const *cad, cudaStream_t st) {
-    return line::launch_add<float>(dp, y, cad, dp.line_tab32.ptr, st);
+bool launch_add_line(DevicePlan &dp, float *y, float const *cad, uint16_t const *colIndex, cudaStream_t st) {
+    return line::launch_add<float>(dp, y, cad, colIndex, dp.line_tab32.ptr, st);
 }
 
 } // namespace a43g

@@ -10,8 +10,8 @@ bool launch_project_line(DevicePlan &dp, double *apc, double const *x, void cons
     return line::launch_project<double>(dp, apc, x, tab, sc, st);
 }
 
-bool launch_add_line(DevicePlan &dp, double *y, double const *cad, cudaStream_t st) {
-    return line::launch_add<double>(dp, y, cad, dp.line_tab64.ptr, st);
+bool launch_add_line(DevicePlan &dp, double *y, double const *cad, uint16_t const *colIndex, cudaStream_t st) {
+    return line::launch_add<double>(dp, y, cad, colIndex, dp.line_tab64.ptr, st);
 }
 
 } // namespace a43g

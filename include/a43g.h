@@ -147,7 +147,8 @@ int a43g_plan_upload(a43g_plan_t *plan);
 
 /* ---- the operator: replaces green_action::action_t<real_t,2,1,64>::multiply
  * (include/green_action.hxx:140-176).  y and x are device pointers to real_t[nnzb][2][64][64];
- * colIndex is the device array [nnzb] of block columns (as the reference passes it);
+ * colIndex is the device array [nnzb] of block columns (as the reference passes it), each below nCols;
+ * the addition of the projectors takes its coefficients by it, all else follows the plan;
  * nnzb and nCols must match the plan; l2nX is accepted for interface compatibility.
  * flops (optional) receives the reference's flop count of one application. */
 int a43g_action_multiply(a43g_plan_t *plan, void *y, const void *x, const uint16_t *colIndex,

@@ -45,13 +45,14 @@ def plan_and_inputs(g, seed=3):
     return p, x, oracle.RestatedOracle(p.export(), Vc, E).action(x)
 
 
-def apply(p, x_np, dtype, offset=0):
+def apply(p, x_np, dtype, offset=0, columns=None):
     t = getattr(torch, dtype)
     n = x_np.size
     buf = [torch.zeros(n + offset, dtype=t, device="cuda") for _ in range(2)]
     x, y = (b[offset:].view(x_np.shape) for b in buf)
     x.copy_(torch.from_numpy(x_np))
-    ci = torch.from_numpy(p.export()["colindx"].astype(np.int16)).cuda()
+    columns = p.export()["colindx"] if columns is None else columns
+    ci = torch.from_numpy(columns.astype(np.int16)).cuda()
     green_action.action_t(p, dtype).multiply(y, x, ci, p.nnzb, p.nCols)
     torch.cuda.synchronize()
     return y.double().cpu().numpy()
@@ -100,3 +101,20 @@ def test_longest_lines(nz, dtype):
     p, x, ref = plan_and_inputs(geometry((2, 1, nz), (1, 1, 1), 80.0, (1, 1, 1), 4, 0))
     assert p.nnzb == 2 * nz
     assert rel_err(apply(p, x, dtype), ref) < TOL[dtype]
+
+
+@pytest.mark.parametrize("dtype", sorted(TOL))
+@pytest.mark.parametrize("name", ["wide", "mixed_to_5", "mixed_to_7"])
+def test_addition_reads_the_callers_columns(name, dtype):
+    """The addition takes the coefficients of the columns that the caller names: here any source for
+    any block, so that the cubes of a segment take different ones."""
+    g = GEOMETRIES[name]()
+    Vc, mats, offs, E, k, dVol, _ = inputs_for(g)
+    p = product_plan(g, Vc, mats, offs, E, k, dVol)
+    rng = np.random.default_rng(8)
+    x = rng.standard_normal((p.nnzb, 2, 64, 64))
+    e = p.export()
+    e["colindx"] = rng.integers(0, p.nCols, p.nnzb).astype(e["colindx"].dtype)
+    ref = oracle.RestatedOracle(e, Vc, E).action(x)
+    assert rel_err(ref, oracle.RestatedOracle(p.export(), Vc, E).action(x)) > 1e-3
+    assert rel_err(apply(p, x, dtype, columns=e["colindx"]), ref) < TOL[dtype]
