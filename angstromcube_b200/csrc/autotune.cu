@@ -1,10 +1,11 @@
 // Autotuner of the action's schedule for one plan on the current device.
 //
 // The kernels have a few schedule parameters whose best value depends on the plan (how many
-// blocks, how many atom images per block, how long the z-lines are) and on the GPU:
-//   * prj_chunk   : blocks of one (image, source) list per projection CTA (the cubes-per-CTA
-//                   schedule of the projection: longer chunks amortize the start and the
-//                   partial sums, shorter ones balance the load)   {12, 24, 40}
+// blocks, how many atom images per block) and on the GPU:
+//   * prj_chunk   : positions of one (image, source) list per projection CTA (longer chunks amortize
+//                   the start and the partial sums, shorter ones balance the load): what the plan's size
+//                   gives (prj_chunk_by_size, the untuned value), or 12, 24, 40 where that is faster by
+//                   more than the 2 % that such timings differ
 //   * use_tc      : FP32 projector on the tensor cores (3xTF32) or on the CUDA cores
 // Each parameter is tuned in turn (coordinate descent), every candidate timed with CUDA events
 // on the caller's stream: two untimed applications, then the mean of three.  Scratch vectors
@@ -20,13 +21,11 @@ namespace a43g {
 namespace {
 
 template <typename T>
-bool time_part(DevicePlan &dp, int part, T *y, T const *x, uint16_t const *ci, cudaStream_t st, float &ms) {
+bool time_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *ci, cudaStream_t st, float &ms) {
     cudaEvent_t e0, e1;
     A43G_CUDA_TRY(cudaEventCreate(&e0));
     A43G_CUDA_TRY(cudaEventCreate(&e1));
-    auto run = [&]() {
-        return (0 == part) ? launch_local<T>(dp, y, x, st) : launch_dyadic<T>(dp, y, x, ci, st);
-    };
+    auto run = [&]() { return launch_dyadic<T>(dp, y, x, ci, st); };
     bool ok = run() && run();
     if (ok) {
         cudaEventRecord(e0, st);
@@ -57,22 +56,31 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
     char line[160];
     float ms = 0;
     if (dp.nAI > 0 && dp.nCols > 0) {
-        uint32_t best = dp.prj_chunk; float tbest = 1e30f;
-        for (uint32_t c : {12u, 24u, 40u}) {
+        uint32_t best = 0;                          // 0: by the plan's size
+        float tsize = 0, tbest = 0;
+        bool const tc_before = dp.use_tc;
+        dp.use_tc = false;                          // the tensor-core projection reads no work items
+        bool ok = true;
+        for (uint32_t c : {0u, 12u, 24u, 40u}) {
             dp.prj_chunk = c;
-            if (!build_prj_items(hp, dp) || !time_part<T>(dp, 1, y, x, ci, st, ms)) return false;
-            std::snprintf(line, sizeof(line), "projector chunk %2u blocks: %.3f ms\n", c, ms); report += line;
-            if (ms < tbest) { tbest = ms; best = c; }
+            ok = build_prj_items(hp, dp) && time_dyadic<T>(dp, y, x, ci, st, ms);
+            if (!ok) break;
+            std::snprintf(line, sizeof(line), "projector chunk %2u blocks%s: %.3f ms\n", c ? c : prj_chunk_by_size(hp),
+                          c ? "" : " (by the plan's size)", ms);
+            report += line;
+            if (0 == c) tsize = tbest = ms;
+            else if (ms < 0.98f*tsize && ms < tbest) { tbest = ms; best = c; }
         }
+        dp.use_tc = tc_before;
         dp.prj_chunk = best;
-        if (!build_prj_items(hp, dp)) return false;
+        if (!readers_done(st) || !build_prj_items(hp, dp) || !ok) return false;
         if (sizeof(T) == 4) {
             if (tc_projector_supported(dp)) {
                 bool const before = dp.use_tc;
                 float t[2] = {0, 0};
                 for (int tc = 0; tc < 2; ++tc) {
                     dp.use_tc = (1 == tc);
-                    if (!time_part<T>(dp, 1, y, x, ci, st, t[tc])) { dp.use_tc = before; return false; }
+                    if (!time_dyadic<T>(dp, y, x, ci, st, t[tc])) { dp.use_tc = before; return false; }
                     std::snprintf(line, sizeof(line), "projector on the %s: %.3f ms\n", tc ? "tensor cores" : "CUDA cores", t[tc]);
                     report += line;
                 }
@@ -87,7 +95,8 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
         }
     }
     std::snprintf(line, sizeof(line), "chosen: projector chunk %u, local %s, %s projector\n",
-                  dp.prj_chunk, dp.local_rows ? "plain rows" : "pencils", dp.use_tc ? "tensor-core" : "CUDA-core");
+                  dp.prj_chunk ? dp.prj_chunk : prj_chunk_by_size(hp), dp.local_rows ? "plain rows" : "pencils",
+                  dp.use_tc ? "tensor-core" : "CUDA-core");
     report += line;
     A43G_CUDA_TRY(cudaStreamSynchronize(st));
     return true;

@@ -139,6 +139,7 @@ bool readers_done(cudaStream_t st);
 // projection work items (image, source, up to dp.prj_chunk consecutive blocks of its list); no kernel
 // that reads the present ones may be running (readers_done)
 bool build_prj_items(GreenPlan const &hp, DevicePlan &dp);
+uint32_t prj_chunk_by_size(GreenPlan const &hp);
 // a table [slot][order][dir][point] of the plan's slots in the layout of the line kernels
 bool make_line_table(DevicePlan const &dp, double const *slot_H, DeviceBuffer &t64, DeviceBuffer *t32, cudaStream_t st);
 // chooses the schedule parameters of the action for this plan by timing them (autotune.cu)

@@ -219,16 +219,17 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
     return upload_values(hp, dp, nullptr);          // waits for the legacy stream: the tables above too
 }
 
-bool build_prj_items(GreenPlan const &hp, DevicePlan &dp) {
-    constexpr uint32_t kGenericChunk = 16;
+// positions per item: enough items for about 12 CTAs per SM (two CTAs per item at least), since small
+// plans would leave SMs idle, and as many as an item's tables in shared memory allow
+uint32_t prj_chunk_by_size(GreenPlan const &hp) {
     size_t npos = 0;
     for (auto const &c : hp.SHOprj) npos += c.nnz();
-    // positions per item: enough items for about 12 CTAs per SM (two CTAs per item at least), since
-    // small plans would leave SMs idle, and as many as an item's tables in
-    // shared memory allow
-    uint32_t chunk = dp.prj_chunk;
-    if (0 == chunk) chunk = uint32_t(std::min<size_t>(kMaxPrjItem, std::max<size_t>(8, 2*npos/(148*12))));
-    chunk = std::min(chunk, kMaxPrjItem);
+    return uint32_t(std::min<size_t>(kMaxPrjItem, std::max<size_t>(8, 2*npos/(148*12))));
+}
+
+bool build_prj_items(GreenPlan const &hp, DevicePlan &dp) {
+    constexpr uint32_t kGenericChunk = 16;
+    uint32_t const chunk = std::min(dp.prj_chunk ? dp.prj_chunk : prj_chunk_by_size(hp), kMaxPrjItem);
     std::vector<uint32_t> items[8];
     std::vector<PrjItem> line;
     uint32_t groups = 0;

@@ -1521,7 +1521,7 @@ int solve_batched(GreenPlan &hp, DevicePlan &dp, BatchCache &bc, a43g_solve_opti
         if (!err.empty()) { set_error(err); return A43G_ERR_ARGUMENT; }
         bc.dev.reset(new DevicePlan());
         bc.ws.reset(new SolverWorkspace());
-        bc.dev->prj_chunk = dp.prj_chunk;
+        if (1 == wave) bc.dev->prj_chunk = dp.prj_chunk;   // more pairs are more items: by the batch's own size
         if (!upload_plan(bc.host, *bc.dev)) return A43G_ERR_CUDA;
         bc.dev->use_tc = dp.use_tc;
         bc.npairs = wave;

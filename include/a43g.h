@@ -193,8 +193,8 @@ int a43g_action_part(a43g_plan_t *plan, int part, void *y, const void *x, void *
 int a43g_vjp(a43g_plan_t *plan, const void *L, const void *G, double *dV, double *dM, double *dR, void *stream);
 
 /* ---- autotuner (no reference counterpart): times the schedule parameters of the action for
- * this plan in the given precision on the current device (blocks per projection CTA, blocks per
- * addition CTA, local-kernel variant, CUDA-core or tensor-core FP32 projector) and keeps the
+ * this plan in the given precision on the current device (blocks per projection CTA, against what
+ * the plan's size gives without tuning; CUDA-core or tensor-core FP32 projector) and keeps the
  * fastest for the plan's later calls; allocates two scratch block vectors for its duration.
  * report (optional) receives a text summary of the timings. */
 int a43g_plan_autotune(a43g_plan_t *plan, int dtype, void *stream, char *report, size_t report_size);

@@ -300,3 +300,17 @@ def test_autotune_keeps_parity(name):
     assert rel_err(apply(p, x, np.float32), y_ref) < FP32_TOL
     assert "chosen" in green_action.autotune(p, "float64")
     assert rel_err(apply(p, x, np.float64), y_ref) < FP64_TOL
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float64"])
+@pytest.mark.parametrize("name", ["wrap8", "peri_xy_wrap_z"])
+def test_autotune_never_leaves_the_untuned_chunk_for_a_slower_one(name, dtype):
+    """The work-item length of an untuned plan is timed first and kept unless another is faster."""
+    import re
+    g = GEOMETRIES[name]()
+    p = product_plan(g, *inputs_for(g)[:6])
+    report = green_action.autotune(p, dtype)
+    times = re.findall(r"projector chunk +(\d+) blocks( \(by the plan's size\))?: ([0-9.]+) ms", report)
+    assert [bool(t[1]) for t in times] == [True, False, False, False], report
+    chosen = re.search(r"chosen: projector chunk (\d+)", report).group(1)
+    assert chosen == times[0][0] or float(dict((t[0], t[2]) for t in times[1:])[chosen]) < float(times[0][2]), report
