@@ -1073,7 +1073,7 @@ bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, c
     // the tensor-core projection stages x with 16-byte copies; the line kernels take 8-byte lanes of x and
     // y, and vectors on 16 bytes; other vectors take the generic kernels
     bool const aligned16 = vectors_aligned(x, x, 16);
-    bool const tc = (sizeof(T) == 4) && dp.use_tc && aligned16 && tc_projector_supported(dp);
+    bool const tc = (sizeof(T) == 4) && dp.use_tc && dp.slot_H32.ptr && aligned16 && tc_projector_supported(dp);
     bool const lines = !tc && vectors_aligned(x, y, 16);
     if (tc) {
         if (!launch_project_tc(dp, (float const*)x, st)) return false;
@@ -1090,7 +1090,7 @@ bool launch_dyadic(DevicePlan &dp, T *y, T const *x, uint16_t const *colIndex, c
         launch_project_L<T, 6>(dp, x, st); launch_project_L<T, 7>(dp, x, st);
     }
     dim3 const ga = row_grid(dp), gm = mul_grid(dp);
-    if (dp.lmax_max <= 5 && !dp.atom_chain3) {
+    if (one_atom_kernel(dp)) {
         sho_atom_kernel<T><<<dim3(dp.nAtoms, dp.nCols, 2), 32*kAtomWarps, atom_smem(dp.lmax_max), st>>>(dptr<T>(dp.cad), dptr<T>(dp.apc), dp.nCols,
             dptr<int8_t>(dp.atom_lmax), dptr<uint32_t>(dp.sum_start), dptr<uint32_t>(dp.sum_col),
             dptr<uint32_t>(dp.img_starts), dptr<double>(dp.img_phase), dptr<double>(dp.atom_mat),

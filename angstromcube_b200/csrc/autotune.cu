@@ -77,6 +77,7 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
         if (sizeof(T) == 4) {
             if (tc_projector_supported(dp)) {
                 bool const before = dp.use_tc;
+                if (!ensure_tc_tables(hp, dp)) return false;
                 float t[2] = {0, 0};
                 for (int tc = 0; tc < 2; ++tc) {
                     dp.use_tc = (1 == tc);
@@ -91,6 +92,7 @@ bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string 
                     A43G_CUDA_TRY(cudaStreamSynchronize(st));
                     if (flag) dp.use_tc = false;
                 }
+                if (!dp.use_tc) dp.slot_H32.release();
             }
         }
     }

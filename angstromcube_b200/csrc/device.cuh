@@ -88,7 +88,7 @@ struct DevicePlan {
     DeviceBuffer atom_starts, atom_lmax, atom_mat, atom_mat_off;
     DeviceBuffer subset_dev;     // uint32 [nCols] diagonal block of each source column
     DeviceBuffer slot_H, slot_mask, prj_slot, add_slot;   // projector tables per (image, row)
-    DeviceBuffer slot_H32;       // float copy of slot_H for the FP32 kernels
+    DeviceBuffer slot_H32;       // float copy of slot_H for the tensor-core projector (ensure_tc_tables)
     int table_stride = 0;        // doubles per slot in slot_H
     DeviceBuffer dev_error;      // int: first error code recorded by a kernel (0: none)
     bool use_tc = true;          // FP32 projector on the tensor cores (else the CUDA cores)
@@ -118,9 +118,8 @@ struct DevicePlan {
     uint32_t max_src_blocks = 0;
     // scratch of the dyadic part (allocated once per plan, never per call)
     DeviceBuffer apc;            // real_t [ncoeffI*nCols][2][64] image projection coefficients
-    DeviceBuffer aac, cadd;      // double [ncoeffA*nCols][2][64]
+    DeviceBuffer aac, cadd;      // double [ncoeffA*nCols][2][64] of the three-kernel atom chain
     DeviceBuffer cad;            // real_t [ncoeffI*nCols][2][64] image addition coefficients
-    size_t apc_elem_bytes = 0;   // 4 or 8: precision the apc/cad scratch is sized for
 };
 
 bool upload_plan(GreenPlan const &hp, DevicePlan &dp);
@@ -146,6 +145,10 @@ bool make_line_table(DevicePlan const &dp, double const *slot_H, DeviceBuffer &t
 template <typename T>
 bool autotune(GreenPlan const &hp, DevicePlan &dp, cudaStream_t st, std::string &report);
 bool ensure_dyadic_scratch(DevicePlan &dp, size_t elem_bytes);
+// tables of the tensor-core projector: made before use_tc is set, since most plans never use them
+bool ensure_tc_tables(GreenPlan const &hp, DevicePlan &dp);
+// the atom matrices by one kernel (its shared memory holds basis sizes up to 5)
+inline bool one_atom_kernel(DevicePlan const &dp) { return dp.lmax_max <= 5 && !dp.atom_chain3; }
 // partial-sum buffer of the deterministic projection for reals of elem_bytes
 bool ensure_prj_part(DevicePlan &dp, size_t elem_bytes);
 

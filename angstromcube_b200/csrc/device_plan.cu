@@ -157,7 +157,6 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
     if (!build_prj_items(hp, dp)) return false;
     dp.table_stride = (hp.table_lmax + 1)*12;
     if (!put(dp.slot_H, hp.slot_H) || !put(dp.slot_mask, hp.slot_mask)) return false;
-    if (!put(dp.slot_H32, std::vector<float>(hp.slot_H.begin(), hp.slot_H.end()))) return false;
     if (!put(dp.prj_slot, hp.prj_slot) || !put(dp.add_slot, hp.add_slot)) return false;
     {   // tables of the line kernels (FP32: every value twice, a pair of columns) and their records
         dp.nslots = uint32_t(hp.slot_mask.size());
@@ -208,10 +207,14 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
         char const *ac = std::getenv("A43G_ATOM_CHAIN");
         dp.atom_chain3 = (ac && 0 == std::strcmp(ac, "three"));
     }
-    if (!dp.aac.alloc(std::max<size_t>(16, size_t(dp.ncoeffA)*dp.nCols*128*sizeof(double)))) return false;
-    if (!dp.cadd.alloc(std::max<size_t>(16, size_t(dp.ncoeffA)*dp.nCols*128*sizeof(double)))) return false;
-    // coefficient scratch of small plans now (4 MB at most, FP64): the first application of a cell of
-    // 64 blocks would spend 25 times its own time on these allocations
+    if (dp.use_tc && !ensure_tc_tables(hp, dp)) return false;
+    if (!one_atom_kernel(dp) &&
+        (!dp.aac.alloc(std::max<size_t>(16, size_t(dp.ncoeffA)*dp.nCols*128*sizeof(double))) ||
+         !dp.cadd.alloc(std::max<size_t>(16, size_t(dp.ncoeffA)*dp.nCols*128*sizeof(double))))) return false;
+    // A cudaMalloc that the driver's pool cannot serve takes 0.35 ms whatever its size, several times an
+    // application of the small plans whose coefficient scratch is 4 MB or less (64 blocks: 0.06 ms), so
+    // they get theirs here, for FP64.  Larger ones get it in their first application, where its precision
+    // is known: half of it for FP32.
     if (dp.nAI > 0 && 2*size_t(dp.ncoeffI)*dp.nCols*1024 + prj_part_bytes(dp, 8) <= (size_t(4) << 20) &&
         (!ensure_dyadic_scratch(dp, 8) || !ensure_prj_part(dp, 8))) return false;
     dp.uploaded = true;
@@ -322,6 +325,10 @@ bool make_line_table(DevicePlan const &dp, double const *slot_H, DeviceBuffer &t
     count_launch();
     A43G_CUDA_TRY(cudaGetLastError());
     return true;
+}
+
+bool ensure_tc_tables(GreenPlan const &hp, DevicePlan &dp) {
+    return dp.slot_H32.ptr || (put(dp.slot_H32, std::vector<float>(hp.slot_H.begin(), hp.slot_H.end())) && uploads_landed());
 }
 
 bool ensure_prj_part(DevicePlan &dp, size_t elem_bytes) {

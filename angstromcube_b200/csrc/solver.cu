@@ -1523,6 +1523,7 @@ int solve_batched(GreenPlan &hp, DevicePlan &dp, BatchCache &bc, a43g_solve_opti
         bc.ws.reset(new SolverWorkspace());
         if (1 == wave) bc.dev->prj_chunk = dp.prj_chunk;   // more pairs are more items: by the batch's own size
         if (!upload_plan(bc.host, *bc.dev)) return A43G_ERR_CUDA;
+        if (dp.use_tc && !ensure_tc_tables(bc.host, *bc.dev)) return A43G_ERR_CUDA;
         bc.dev->use_tc = dp.use_tc;
         bc.npairs = wave;
     }

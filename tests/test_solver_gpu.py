@@ -151,6 +151,26 @@ def test_solve_batched_matches_individual_solves(precision):
         assert true_residual(p, we, X.cpu().numpy()) <= 2e-10
 
 
+def test_solve_batched_on_the_tensor_core_projector(monkeypatch):
+    """A batch takes the one-pair plan's choice of the tensor-core projector and makes the tables that
+    only this projector reads: the densities are those of the CUDA cores to the solves' tolerance."""
+    w = workloads.make("periodic4_1atom")
+    rho = []
+    for projector in ("tc", "simt"):
+        monkeypatch.setenv("A43G_PROJECTOR", projector)
+        p = gf.construct_Green_function(w.geometry)
+        gf.update_potential(p, w.Vcell, w.mats, w.offsets, layout="cells")
+        p.upload()
+        monkeypatch.delenv("A43G_PROJECTOR")
+        stats, r = green_action.solve_batched(p, [complex(-0.4, 0.2), complex(-0.2, 0.3)], np.zeros((2, 3)), w.dVol,
+                                              want_rho=True, batch=2, stream=torch.cuda.Stream(), tolerance=1e-10,
+                                              max_iterations=2000, precision="float32")
+        assert all(s["converged"] for s in stats), stats
+        rho.append(r)
+    assert np.abs(rho[0] - rho[1]).max() <= 1e-8 * np.abs(rho[1]).max()
+    assert not np.array_equal(rho[0], rho[1])
+
+
 def test_solve_concurrent_matches_sequential():
     """Batched solves of several (E, k) pairs on worker plans and streams give the densities of
     the same solves done one after the other."""
