@@ -44,12 +44,11 @@ def test_action_fp64_fp32_vs_oracle(name):
     assert rel_err(y32, y_ref) < FP32_TOL
 
 
-@pytest.mark.parametrize("variant", ["rows", "plain", "pencils", "staged"])
+@pytest.mark.parametrize("variant", ["rows", "pencils"])
 @pytest.mark.parametrize("name", sorted(GEOMETRIES))
 def test_action_fp32_local_variants_vs_oracle(name, variant, monkeypatch):
-    """Every FP32 local kernel (rows with loads ahead; plain rows; y-pencils, the default;
-    y-pencils with staged neighbour cubes) matches the oracle on every boundary condition, with
-    Bloch phases (k != 0)."""
+    """Both FP32 local kernels (pencils, the default; rows, that of z-lines beyond the pencils' limit)
+    match the oracle on every boundary condition, with Bloch phases (k != 0)."""
     g = GEOMETRIES[name]()
     Vc, mats, offs, E, k, dVol, na = inputs_for(g)
     monkeypatch.setenv("A43G_LOCAL", variant)
@@ -59,18 +58,15 @@ def test_action_fp32_local_variants_vs_oracle(name, variant, monkeypatch):
     assert rel_err(apply(p, x, np.float32), y_ref) < FP32_TOL
 
 
-@pytest.mark.parametrize("variant", ["rows", "pencils", "rolled", "chain3"])
+@pytest.mark.parametrize("variant", ["rows", "pencils", "chain3"])
 @pytest.mark.parametrize("name", sorted(GEOMETRIES))
 def test_action_fp64_local_variants_vs_oracle(name, variant, monkeypatch):
-    """Both FP64 local kernels (rows; pencils with the two planes on two threads, the default),
-    both FP64 additions (z-orders unrolled, the default; "rolled": one at a time) and both
-    atom-matrix chains (one kernel, the default; "chain3": collect, multiply, broadcast) match the
-    oracle (FP64 to 1e-12, FP32 to 3e-5) on every boundary condition, with Bloch phases (k != 0)."""
+    """Both FP64 local kernels (pencils, the default; rows) and both atom-matrix chains (one kernel,
+    the default; "chain3": collect, multiply, broadcast) match the oracle (FP64 to 1e-12, FP32 to
+    3e-5) on every boundary condition, with Bloch phases (k != 0)."""
     g = GEOMETRIES[name]()
     Vc, mats, offs, E, k, dVol, na = inputs_for(g)
-    if variant == "rolled":
-        monkeypatch.setenv("A43G_ADD64", "rolled")
-    elif variant == "chain3":
+    if variant == "chain3":
         monkeypatch.setenv("A43G_ATOM_CHAIN", "three")
     else:
         monkeypatch.setenv("A43G_LOCAL64", variant)
