@@ -153,6 +153,8 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
         dp.img_group[L].count = uint32_t(imgs.size());
         if (!put(dp.img_group[L].images, imgs)) return false;
     }
+    // positions per projection work item: by the plan's size (default) or a given number
+    if (char const *c = std::getenv("A43G_PRJ_CHUNK")) dp.prj_chunk = uint32_t(std::max(0, std::atoi(c)));
     if (dp.lmax_max > 7) { set_error("projector basis sizes above numax 7 are not supported"); return false; }
     if (!build_prj_items(hp, dp)) return false;
     dp.table_stride = (hp.table_lmax + 1)*12;

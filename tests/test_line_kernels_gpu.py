@@ -66,6 +66,20 @@ def test_action_at_the_edges(name, dtype):
     assert np.array_equal(apply(p, x, dtype), apply(p, x, dtype))      # sums in a fixed order
 
 
+@pytest.mark.parametrize("chunk", [1, 2, 39, 40, 41])
+@pytest.mark.parametrize("name", ["wide", "mixed_to_7"])
+def test_work_items_of_every_length(name, chunk, monkeypatch):
+    """Projection items of one position, of the most that fit an item's tables (40; 41 is cut to it) and
+    lists that they divide unevenly."""
+    monkeypatch.setenv("A43G_PRJ_CHUNK", str(chunk))
+    p, x, ref = plan_and_inputs(GEOMETRIES[name]())
+    lengths = np.diff(p.export()["SHOprj_start"].reshape(p.nCols, -1), axis=1)
+    assert lengths.max() > 41 and (lengths % min(chunk, 40) != 0).any() == (chunk > 1)
+    for dtype in TOL:
+        assert rel_err(apply(p, x, dtype), ref) < TOL[dtype]
+        assert np.array_equal(apply(p, x, dtype), apply(p, x, dtype))
+
+
 @pytest.mark.parametrize("dtype", sorted(TOL))
 def test_vectors_off_the_16_byte_boundary(dtype):
     """One element further, x and y take the projector kernels without 16-byte copies."""

@@ -323,6 +323,26 @@ def test_preconditioned_solve_same_solution_fewer_iterations(precision):
     assert true_residual(p, we, X.cpu().numpy()) <= 1e-8
 
 
+@pytest.mark.parametrize("precision", ["float64", "float32"])
+def test_preconditioner_on_an_odd_number_of_blocks(precision):
+    """27 blocks leave half of the FP32 preconditioner's last CTA without work; the solution has the
+    true residual and the densities of the plain solve."""
+    from helpers import geometry, inputs_for, product_plan
+    g = geometry((3, 3, 3), (1, 1, 1), 6.0, (1, 1, 1), 4, 2)
+    Vc, mats, offs, _, k, dVol, _ = inputs_for(g)
+    E = complex(-0.4, 0.3)
+    p = product_plan(g, Vc, mats, offs, E, k, dVol)
+    assert p.nnzb == 27
+    opts = dict(tolerance=1e-9, max_iterations=2000, precision=precision, stream=torch.cuda.Stream())
+    _, rho0 = green_action.solve(p, **opts)
+    X = torch.full((27, 2, 64, 64), float("nan"), device="cuda", dtype=torch.float64)
+    st, rho = green_action.solve(p, X=X, precondition=True, **opts)
+    assert st["residual_max"] <= 1e-8, st
+    assert np.abs(rho - rho0).max() <= 1e-7 * np.abs(rho0).max()
+    w = workloads.Workload("27 blocks", g, Vc, mats, offs, E, k, dVol, 1e-9, 2000)
+    assert true_residual(p, w, X.cpu().numpy()) <= 1e-8
+
+
 def test_preconditioned_batched_matches_individual():
     """Batched and individual preconditioned solves (each pair with its own energy in the
     preconditioner's scaling) give the same densities."""

@@ -228,3 +228,18 @@ def test_vjp_matches_reference_cpu_solves():
     Lcu = torch.from_numpy(Lr).cuda()
     dR_ref = green_action.vjp(p, Lcu, Gcu, potential=False, matrices=False)["R"]
     assert np.abs(out_gpu["R"] - dR_ref).max() <= 1e-7 * np.abs(dR_ref).max()
+
+
+@pytest.mark.parametrize("call", ["vjp", "density"])
+@pytest.mark.parametrize("numax,mixed", [(0, False), (1, False), (2, False), (4, False), (5, True), (6, False), (7, False), (7, True)])
+def test_basis_sizes_vs_dense_projectors(call, numax, mixed):
+    """Gradients and density matrices of every padding of the (differentiated) tables, against the same
+    sums with the projectors as dense matrices in 64 bits (perf/cases.py).  Every value is a sum of at
+    most a few 10,000 products: 1e-11 is some 50,000 roundings."""
+    from perf import cases
+    case = cases._case(call, (4, 5, 3), (1, 2, 1), bc="111" if call == "vjp" else "000", atoms=7 if mixed else 3, numax=numax,
+                       mixed=mixed, lattice=False, r_trunc=3.0, kx=0.1, ky=0.2, kz=-0.15)
+    out, ref = cases.run(cases.prepare(case, 5)), cases.exact(case, 5)
+    for a, b in zip(out if call == "vjp" else [out], ref if call == "vjp" else [ref]):
+        assert a.shape == b.shape and np.abs(b).max() > 0
+        assert np.abs(a - b).max() <= 1e-11 * np.abs(b).max()
