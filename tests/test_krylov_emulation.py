@@ -6,8 +6,10 @@ import numpy as np
 import pytest
 
 import krylov_emulation as ke
+import oracle
 
-pytestmark = pytest.mark.timeout(600)
+pytestmark = [pytest.mark.timeout(600),
+              pytest.mark.skipif(not oracle.ref_available(), reason="oracle/_ref not built")]
 
 
 def test_cocg_at_gamma():
