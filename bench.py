@@ -307,14 +307,11 @@ def read_traffic(kernel):
 
 
 def local_kernel_of(tune_lines):
-    """Name of the FP32 local kernel the autotuner chose (from its "chosen: ..." line) and the key
+    """Name of the FP32 local kernel of the plan (from the autotuner's "chosen: ..." line) and the key
     of its DRAM traffic in profiles/traffic.txt (None where no capture exists)."""
-    chosen = " ".join(tune_lines)
-    if "local pencils" in chosen:
-        return "local_pencil_kernel (FP32 y-pencils: potential + 8th-order kinetic, one pass)", "local_pencil_kernel_f32"
-    if "local plain rows" in chosen:
+    if "local plain rows" in " ".join(tune_lines):
         return "local_fused_kernel<float,16> (potential + 8th-order kinetic, one pass)", None
-    return "local_fused_pf_kernel<float,16> (potential + 8th-order kinetic, one pass)", "local_fused_pf_kernel_f32"
+    return "local_pencil_kernel<float> (potential + 8th-order kinetic, one pass)", "local_pencil_kernel_f32"
 
 
 def check_one_plan(w, pairs):
@@ -485,7 +482,6 @@ def measure_kernels(plan, stream, out, hbm, bf16, peak_kind):
     nsho = 56
     L = 5
     sf_flops = 2.0 * 2 * (64 * (L + 1) + 16 * (L + 1) * (L + 2) // 2 + 4 * nsho) * 128 * plan.sizes["SHOadd_nnz"]
-    fma_peak = 148 * 128 * 2 * 1.965 / 1e3    # TFLOP/s: SMs x FP32 lanes x 2 flops x GHz
     flops = 4.0 * nsho * 64 * 128 * plan.sizes["SHOadd_nnz"]
     tf32_peak = bf16 / 2
     tc = os.environ.get("A43G_PROJECTOR", "") == "tc"
@@ -497,12 +493,12 @@ def measure_kernels(plan, stream, out, hbm, bf16, peak_kind):
                                  "peak_kind": "dense TF32 = half of the %s bf16 peak" % peak_kind,
                                  "algorithmic_flops_per_launch": flops, "ms_per_launch": t_dyadic * 1e3,
                                  "note": "flops of the dense contraction P (64 x 64 per block and image) x X (64 x 128)",
-                                 # the kernels do the sum-factorized work: 64 (L+1) + 16 (L+1)(L+2)/2 + 4 nSHO
-                                 # FMAs per column and (image, block) pair, for the projection and the addition
-                                 "sum_factorized_flops_per_launch": sf_flops,
-                                 "sum_factorized_tflops": sf_flops / t_dyadic / 1e12,
-                                 "fp32_fma_peak_tflops": fma_peak,
-                                 "fp32_fma_frac": sf_flops / t_dyadic / 1e12 / fma_peak}
+                                 # 64 (L+1) + 16 (L+1)(L+2)/2 + 4 nSHO FMAs per column and (image, block) pair,
+                                 # projection and addition: every block contracted by itself.  A measure of
+                                 # the work that is done, not of what the kernels execute: they share the y-
+                                 # and z-contractions along lines of cubes
+                                 "block_equivalent_flops_per_launch": sf_flops,
+                                 "block_equivalent_tflops": sf_flops / t_dyadic / 1e12}
     x64 = torch.randn((nnzb, 2, 64, 64), device="cuda", dtype=torch.float64)
     y64 = torch.empty_like(x64)
     del x, y

@@ -13,23 +13,39 @@ def load_bench():
     return m
 
 
-def test_traffic_table_has_the_local_kernels():
+def test_traffic_table_names_kernels_that_exist():
+    """Every row is a kernel of the sources with its precision, moves at least its vectors (read once,
+    written once) and is the committed capture's figure of the 4,096 blocks."""
     b = load_bench()
-    assert b.read_traffic("local_pencil_kernel_f32") == 66275
-    assert b.read_traffic("local_fused_pf_kernel_f32") == 70326
-    assert b.read_traffic("local_pencil64_kernel_f64") == 159058
+    with open(os.path.join(ROOT, "angstromcube_b200", "csrc", "action.cu")) as f:
+        source = f.read()
+    with open(os.path.join(ROOT, "profiles", "ncu_action_one_source.md")) as f:
+        rows = [[c.strip(" `") for c in line.split("|")[1:-1]] for line in f if line.startswith("| ")]
+    head, traffic = rows[0], next(r for r in rows if r[0].startswith("DRAM traffic"))
+    keys = [k for k in ("local_pencil_kernel_f32", "local_pencil_kernel_f64") if b.read_traffic(k) is not None]
+    with open(os.path.join(ROOT, "profiles", "traffic.txt")) as f:
+        assert keys == [line.split()[0] for line in f if line.strip() and not line.startswith("#")]
+    for key in keys:
+        name, precision = key[:-4], key[-3:]
+        assert name + "(" in source
+        per_block = b.read_traffic(key)
+        assert per_block >= 2 * 8192 * int(precision[1:]) / 8
+        captured = float(traffic[head.index("local_pencil " + precision.upper().replace("F", "FP"))]) * 1e6 / 4096
+        assert abs(per_block - captured) < 100            # the table gives 0.1 MB
     assert b.read_traffic("no_such_kernel") is None
 
 
 def test_local_kernel_named_from_the_autotuner_choice():
     b = load_bench()
-    line = ["chosen: projector chunk 32, addition 8 blocks per CTA, local %s, CUDA-core projector"]
-    name, key = b.local_kernel_of([line[0] % "pencils"])
-    assert name.startswith("local_pencil_kernel") and key == "local_pencil_kernel_f32"
-    name, key = b.local_kernel_of([line[0] % "rows with loads ahead"])
-    assert name.startswith("local_fused_pf_kernel") and key == "local_fused_pf_kernel_f32"
-    name, key = b.local_kernel_of([line[0] % "plain rows"])
+    line = "chosen: projector chunk 40, local %s, CUDA-core projector"
+    name, key = b.local_kernel_of([line % "pencils"])
+    assert name.startswith("local_pencil_kernel<float>") and key == "local_pencil_kernel_f32"
+    name, key = b.local_kernel_of([line % "plain rows"])
     assert name.startswith("local_fused_kernel") and key is None
+    with open(os.path.join(ROOT, "angstromcube_b200", "csrc", "autotune.cu")) as f:
+        source = f.read()                                 # the line is the autotuner's
+    assert 'chosen: projector chunk %u, local %s, %s projector' in source
+    assert '"plain rows" : "pencils"' in source
 
 
 def test_pair_walk_is_a_permutation_spread_over_the_contour():
