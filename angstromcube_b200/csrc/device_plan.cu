@@ -201,7 +201,7 @@ bool upload_plan(GreenPlan const &hp, DevicePlan &dp) {
         // FP32 projector: CUDA cores (default) or the tensor cores ("tc"); FP64 always on the CUDA cores
         char const *e = std::getenv("A43G_PROJECTOR");
         dp.use_tc = (e && 0 == std::strcmp(e, "tc"));
-        // local kernel: pencils (default) or "rows" ("plain" in FP32), the kernel of unaligned vectors
+        // local kernel: pencils (default) or "rows" (also "plain"), the kernel of lines beyond the pencils' limit
         char const *l = std::getenv("A43G_LOCAL"), *l64 = std::getenv("A43G_LOCAL64");
         dp.local_rows = (l && (0 == std::strcmp(l, "rows") || 0 == std::strcmp(l, "plain"))) ||
                         (l64 && 0 == std::strcmp(l64, "rows"));

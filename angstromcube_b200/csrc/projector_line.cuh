@@ -6,10 +6,12 @@
 //     P_(ix,iy,iz)(x, y, z) = H_ix(x) H_iy(y) H_iz(z)   for points inside the projection radius,
 // and so is the whole sphere: all cubes of one x-line share H_iy(y) and H_iz(z), all lines of one
 // z-slab of cubes share H_iz(z).  The x-contraction of the projection therefore accumulates over a whole line
-// before the y-contraction is done once per line, and the z-contraction once per slab: with about
-// 6 cubes per line and 36 per slab a block costs 64(L+1) + 16 N2/6 + 4 nSHO/36 multiply-adds per
-// column (about 450 at L = 5, N2 = (L+1)(L+2)/2) instead of 64(L+1) + 16 N2 + 4 nSHO (944) when every
-// block is contracted by itself, and 3584 for the dense product.
+// before the y-contraction is done once per line, and the z-contraction once per slab.  In the cells in
+// use a line has 2.5 to 4.5 cubes (whole spheres about 6; images are cut by the faces of cells and
+// truncation spheres) and is cut where a work item ends, so that 2.1 to 4.2 blocks share a y-contraction
+// and 4 to 16 a z-contraction: 480 to 600 multiply-adds per block and column at L = 5 (480 on the
+// 64-atom cell) instead of 64(L+1) + 16 N2 + 4 nSHO = 944, N2 = (L+1)(L+2)/2, when every block is
+// contracted by itself, and 3584 for the dense product.
 #pragma once
 
 #include "device.cuh"
@@ -380,8 +382,8 @@ __device__ __noinline__ void add_by_columns(T *yl, T const *cq, uint32_t nrhs, u
 //
 // Measured on the 64-atom cell with 8 sources, against one contraction per (block, image) pair:
 // FP32 1.91 -> 0.93 ms, FP64 3.86 -> 1.87 ms (1.02 and 2.07 ms with y staged in shared memory from
-// the start of the CTA on).  The FP64 pipe is about a third busy (issue slots too): the point sums
-// take 128 of the 244 registers, which leaves two CTAs per SM.  Segments of 2 cubes and three CTAs
+// the start of the CTA on).  The FMA pipe is about a third busy (issue slots too): the point sums
+// take 128 of some 250 registers, which leaves two CTAs per SM.  Segments of 2 cubes and three CTAs
 // per SM are 2 % slower there, and two records per barrier no faster.
 template <typename T, int LMAX, int SEG>
 __global__ void __launch_bounds__(kThreads, LMAX <= 5 ? 2 : 1)
