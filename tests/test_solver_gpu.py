@@ -171,6 +171,32 @@ def test_solve_batched_on_the_tensor_core_projector(monkeypatch):
     assert not np.array_equal(rho[0], rho[1])
 
 
+@pytest.mark.parametrize("precision", ["float64", "float32"])
+def test_retirement_with_many_work_items_per_source(precision, monkeypatch):
+    """Sources that retire one after the other while every (image, source) pair has an item per block:
+    the same solution as without retirement, and afterwards the plan's action is that of a fresh plan
+    (no item of a retired source has taken a ticket)."""
+    monkeypatch.setenv("A43G_PRJ_CHUNK", "1")
+    w, p = setup("periodic8_8atoms_s2x2x1")
+    gf.update_energy_parameter(p, complex(-0.3, 0.25), w.dVol)
+    opts = dict(tolerance=1e-9, max_iterations=3000, precision=precision, check_every=1, stream=torch.cuda.Stream())
+    X = [torch.zeros((p.nnzb, 2, 64, 64), device="cuda", dtype=torch.float64) for _ in range(2)]
+    for x, retire in zip(X, (True, False)):
+        st, _ = green_action.solve(p, X=x, retire=retire, **opts)
+        assert st["residual_max"] <= 1e-8, st
+    torch.cuda.synchronize()
+    assert torch.equal(*X)
+    _, fresh = setup("periodic8_8atoms_s2x2x1")
+    gf.update_energy_parameter(fresh, complex(-0.3, 0.25), w.dVol)
+    ci = torch.from_numpy(p.export()["colindx"].astype(np.int16)).cuda()
+    y = []
+    for q in (p, fresh):
+        y.append(torch.empty_like(X[0], dtype=getattr(torch, precision)))
+        green_action.action_t(q, precision).multiply(y[-1], X[0].to(y[-1].dtype), ci, q.nnzb, q.nCols)
+    torch.cuda.synchronize()
+    assert torch.equal(*y)
+
+
 def test_solve_concurrent_matches_sequential():
     """Batched solves of several (E, k) pairs on worker plans and streams give the densities of
     the same solves done one after the other."""
